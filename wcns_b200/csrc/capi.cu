@@ -101,6 +101,7 @@ struct WcnsContext {
     SaFields SA{};
     SaParams SAP{};
     int launches = 0;
+    bool clustered = false;  // the blocks fit the clustered sweeps
     std::unique_ptr<WideSweep> wide;
     std::vector<DevWall> hwalls;  // host copy of the wall table (block order)
     double *adj_pool = nullptr;   // the adjoint slots (WCNS_ADJ_*), five fields each, on first use
@@ -258,6 +259,15 @@ static void free_owned(WcnsContext *c, void *p) {
     cudaFree(p);
 }
 
+// Contexts whose blocks have at most this many hyperplanes sweep clustered by
+// default, the shape that they have always reported.  It is not the faster
+// form any more, but close: 0.149 against 0.129 ms per step on the small plate
+// (35 planes, eight blocks), and the autotuner chooses.  Above, the wide
+// sweeps are the default (33x17x9: 0.176 against 0.209 ms; 65x33x17: 0.34
+// against 0.57; the 228,888-point plate: 0.61 against 0.85; the 64-case batch:
+// 0.55 against 2.25).
+constexpr int SWEEP_SMALL_PLANES = 35;
+
 // The wide cooperative sweeps' chunks and arrays (and the SA model's when it
 // is set up); L.wide points to them.  -1: the blocks cannot be swept wide;
 // a CUDA error code when an allocation fails.
@@ -270,35 +280,61 @@ static int wide_alloc(WcnsContext *c) {
     auto W = std::make_unique<WideSweep>();
     if (setup_sweep_wide(L, *W) != 0) return -1;
     WideArrays &A = W->A;
-    const size_t words = (size_t)(WIDE_COEF_WORDS + 5 + 5 + 15 + 5) * A.n + 8;
-    CK(cudaMalloc(&A.stat, sizeof(double) * words));
-    c->owned.push_back(A.stat);
-    A.rhs = A.stat + (size_t)WIDE_COEF_WORDS * A.n;
-    A.dql = A.rhs + (size_t)5 * A.n;
-    A.gs1 = A.dql + (size_t)5 * A.n;
-    A.gs2 = A.gs1 + (size_t)15 * A.n;
-    CK(cudaMalloc(&A.ring, sizeof(double) * (size_t)std::max(1, A.nbnd) * 8 * A.nkmax * 10));
+    CK(cudaMalloc(&A.rec, sizeof(double2) * WIDE_PAIRS * (size_t)A.n));
+    c->owned.push_back(A.rec);
+    // ring, the readers' counts and the tag base, all zero: tags start above
+    const size_t ring = (size_t)16 * WIDE_UNITS * A.ringn * A.nkmax * std::max(1, A.nbnd), fl = sizeof(unsigned) * (size_t)(A.nbnd + 1);
+    CK(cudaMalloc(&A.ring, ring));
     c->owned.push_back(A.ring);
-    CK(cudaMalloc(&A.flags, sizeof(unsigned) * 2 * (size_t)std::max(1, A.nbnd)));
+    CK(cudaMemset(A.ring, 0, ring));
+    CK(cudaMalloc(&A.flags, fl));
     c->owned.push_back(A.flags);
+    CK(cudaMemset(A.flags, 0, fl));
+    A.epoch = A.flags + A.nbnd;
     if (c->sa_pool) {  // the model's scalar sweeps run on the wide chunks too
-        CK(cudaMalloc(&A.sa, sizeof(double) * (6 * (size_t)A.n + 8)));
+        CK(cudaMalloc(&A.sa, sizeof(double2) * WIDE_SA_PAIRS * (size_t)A.n));
         c->owned.push_back(A.sa);
     }
-    W->chunks = c->up(W->hchunks);
+    W->ctas = c->up(W->hctas);
+    W->segs = c->up(W->hsegs);
     c->wide = std::move(W);
     L.wide = c->wide.get();
+    return 0;
+}
+
+// The clustered sweeps' arrays, plane-major: dq (5 planes of values), the
+// static records (SR_N per cell) and three dynamic records (DYN_N per cell);
+// the memset leaves zero the records that no kernel ever writes.  A context
+// that sweeps wide has them from the first time that a cluster shape is asked
+// for.
+static int pm_alloc(WcnsContext *c) {
+    if (c->pm_pool) return 0;
+    const size_t pmbytes = sizeof(double) * (size_t)(5 + SR_N + 3 * DYN_N) * (size_t)c->total_pm;
+    if (cudaMalloc(&c->pm_pool, pmbytes) != cudaSuccess) {
+        c->pm_pool = nullptr;
+        cudaGetLastError();
+        set_err("device allocation of the sweep arrays failed");
+        return WCNS_ERR_CUDA;
+    }
+    CK(cudaMemset(c->pm_pool, 0, pmbytes));
+    for (int m = 0; m < 5; m++) c->PM.dq[m] = c->pm_pool + (size_t)m * c->total_pm;
+    c->PM.dq_stride = c->total_pm;
+    c->PM.stat = c->pm_pool + (size_t)5 * c->total_pm;
+    c->PM.dyn = c->PM.stat + (size_t)SR_N * c->total_pm;
+    c->PM.gs[0] = c->PM.dyn + (size_t)DYN_N * c->total_pm;
+    c->PM.gs[1] = c->PM.gs[0] + (size_t)DYN_N * c->total_pm;
     return 0;
 }
 
 static void wide_free(WcnsContext *c) {
     if (!c->wide) return;
     WideSweep &W = *c->wide;
-    free_owned(c, W.A.stat);
+    free_owned(c, W.A.rec);
     free_owned(c, W.A.ring);
     free_owned(c, W.A.flags);
     free_owned(c, W.A.sa);
-    free_owned(c, W.chunks);
+    free_owned(c, W.ctas);
+    free_owned(c, W.segs);
     c->wide.reset();
     c->L.wide = nullptr;
 }
@@ -619,12 +655,24 @@ static int build_tables(WcnsContext *c) {
         int cl = 16, fine = 1;
         if (const char *e = getenv("WCNS_SWEEP_CLUSTER")) cl = atoi(e);
         if (const char *e = getenv("WCNS_SWEEP_FINE")) fine = atoi(e);
-        // blocks whose columns do not fit the clustered kernel run the wide
-        // cooperative sweeps, or, when those do not fit either, sweep plane by plane
+        // The wide cooperative sweeps, except where every block has at most
+        // SWEEP_SMALL_PLANES hyperplanes or the wide ones do not fit: there the
+        // clustered kernel (one cluster per block) where its shared memory holds
+        // the blocks' columns, else plane by plane
         const bool want_plane = c->prm.flags & WCNS_FLAG_SWEEP_BY_PLANE, want_wide = c->prm.flags & WCNS_FLAG_SWEEP_WIDE;
         const bool clustered = !want_plane && !want_wide && setup_sweep(L, cl, fine) == 0;
-        if (!clustered && !want_plane)
-            if (int rc = wide_alloc(c); rc > 0) return rc;
+        c->clustered = clustered;
+        int planes = 0;
+        for (int b = 0; b < nbk; b++) planes = std::max(planes, c->blk[b].d.ni + c->blk[b].d.nj + c->blk[b].d.nk - 2);
+        const bool prefer_wide = !clustered || (planes > SWEEP_SMALL_PLANES && !getenv("WCNS_SWEEP_CLUSTER"));
+        if (prefer_wide && !want_plane) {
+            const size_t had = c->owned.size();
+            if (int rc = wide_alloc(c); rc > 0) {
+                while (c->owned.size() > had) free_owned(c, c->owned.back());
+                if (!clustered) return rc;  // no memory, and no other form
+                cudaGetLastError();
+            }
+        }
         L.sweep_plane = !clustered && !L.wide ? 1 : 0;
     }
     // residual partials, update bad lists
@@ -797,20 +845,8 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
     }
     rc = build_tables(c);
     if (rc) { delete c; return rc; }
-    if (!L.sweep_plane && !L.wide) {
-        // sweep arrays, plane-major: dq (5 planes of values), the static records
-        // (SR_N per cell) and three dynamic records (DYN_N per cell); the memset
-        // leaves zero the records that no kernel ever writes
-        size_t pmbytes = sizeof(double) * (size_t)(5 + SR_N + 3 * DYN_N) * (size_t)c->total_pm;
-        if (cudaMalloc(&c->pm_pool, pmbytes) != cudaSuccess) { delete c; set_err("device allocation of the sweep arrays failed"); return WCNS_ERR_CUDA; }
-        cudaMemset(c->pm_pool, 0, pmbytes);
-        for (int m = 0; m < 5; m++) c->PM.dq[m] = c->pm_pool + (size_t)m * c->total_pm;
-        c->PM.dq_stride = c->total_pm;
-        c->PM.stat = c->pm_pool + (size_t)5 * c->total_pm;
-        c->PM.dyn = c->PM.stat + (size_t)SR_N * c->total_pm;
-        c->PM.gs[0] = c->PM.dyn + (size_t)DYN_N * c->total_pm;
-        c->PM.gs[1] = c->PM.gs[0] + (size_t)DYN_N * c->total_pm;
-    }
+    if (!L.sweep_plane && !L.wide)
+        if (int rc2 = pm_alloc(c)) { delete c; return rc2; }
     c->PM.csize = L.sweep_cluster;
     CK(cudaMalloc(&c->d_err, sizeof(int) * ERR_NSLOTS));
     c->owned.push_back(c->d_err);
@@ -1178,7 +1214,7 @@ extern "C" int wcns_sa_setup(WcnsContext *c, const double *const *xyz, double ti
     if (c->L.wide && !c->L.wide->A.sa) {
         // the model's scalar sweeps run on the wide chunks too
         WideArrays &A = c->L.wide->A;
-        CK(cudaMalloc(&A.sa, sizeof(double) * (6 * (size_t)A.n + 8)));
+        CK(cudaMalloc(&A.sa, sizeof(double2) * WIDE_SA_PAIRS * (size_t)A.n));
         c->owned.push_back(A.sa);
     }
     // the mean-flow kernels now read vist (spectvist, the viscous
@@ -1575,9 +1611,9 @@ extern "C" int wcns_get_shape(WcnsContext *c, int *shape) {
     return 0;
 }
 
-// a context whose blocks fit the clustered sweeps (its plane-major arrays
-// exist) can also sweep wide, and switch between the two
-static bool can_cluster(const WcnsContext *c) { return c->pm_pool != nullptr; }
+// a context whose blocks fit the clustered sweeps can also sweep wide, and
+// switch between the two
+static bool can_cluster(const WcnsContext *c) { return c->clustered; }
 
 static int apply_shape(WcnsContext *c, const int *shape) {
     LaunchCtx &L = c->L;
@@ -1596,6 +1632,7 @@ static int apply_shape(WcnsContext *c, const int *shape) {
                         " CTAs per cluster in that lane mode");
                 return WCNS_ERR_ARGUMENT;
             }
+            if (int rc = pm_alloc(c)) return rc;
             c->PM.csize = L.sweep_cluster;
             wide_free(c);
         }
@@ -1666,7 +1703,7 @@ extern "C" int wcns_autotune(WcnsContext *c, int reps, int *shape, double *ms) {
     wcns_get_shape(c, best);
     double best_ms[3] = {0.0, 0.0, 0.0};
     // the LU-SGS sweep form and shape: every cluster shape, and the wide sweeps
-    if (can_cluster(c) && !L.sweep_plane) {
+    if (can_cluster(c) && !L.sweep_plane && pm_alloc(c) == 0) {
         double tbest = 1e300;
         const bool was_wide = L.wide != nullptr;
         L.wide = nullptr;

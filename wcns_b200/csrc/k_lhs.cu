@@ -11,11 +11,10 @@
 // sequential result exactly.
 //
 // Work split:
-//   k_lhs_prep   (all cells in parallel) evaluates everything that does not
-//                depend on dq -- the coefficients of mxdq_std for the cell
-//                acting as a neighbour (both signs, three directions), coed,
-//                the viscous radii -- and rhs = dq (store_rhs_nb), as one
-//                packed 368-byte record per cell in plane-major order.
+//   k_lhs_prep   (all cells in parallel) packs what the sweeps need of a cell
+//                that does not depend on dq -- velocity, total enthalpy,
+//                metrics, radii (wcns_sweep.cuh), coed -- and rhs = dq
+//                (store_rhs_nb) into one 208-byte record in plane-major order.
 //   k_sweep      one thread-block cluster per grid block (the reference's
 //                LU-SGS is block-Jacobi, so blocks are independent).  CTA q
 //                of the cluster owns a j-chunk of the block's (j,k) columns;
@@ -36,6 +35,7 @@
 
 #include "wcns_dev.cuh"
 #include "wcns_launch.h"
+#include "wcns_sweep.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -47,45 +47,6 @@ __global__ void k_zero_faces(DevFields F, const long long *__restrict__ pts, lon
 #pragma unroll
         for (int m = 0; m < 5; m++) F.f[F_DQ1 + m][id] = 0.0;
     }
-}
-
-// mxdq_std (LHS.f90:756-828) split into dq-independent coefficients
-// (k_lhs_prep) and the linear map applied to dq (jac_apply); operations and
-// their order are those of the reference routine.
-struct Jac {
-    double l1, x1, x2, ct, nx, ny, nz, af, um, vm, wm, c2, hm;
-};
-
-__device__ __forceinline__ void jac_apply(const DevParams &P, const Jac &J, const double *dq, double *f) {
-    const double ae = P.gama - 1.0;
-    double dc = J.ct * dq[0] - J.nx * dq[1] - J.ny * dq[2] - J.nz * dq[3];
-    double dh = J.af * dq[0] - ae * (J.um * dq[1] + J.vm * dq[2] + J.wm * dq[3] - dq[4]);
-    double c2dc = J.c2 * dc;
-    f[0] = J.l1 * dq[0] - dh * J.x1 - dc * J.x2;
-    f[1] = J.l1 * dq[1] + (J.nx * c2dc - J.um * dh) * J.x1 + (J.nx * dh - J.um * dc) * J.x2;
-    f[2] = J.l1 * dq[2] + (J.ny * c2dc - J.vm * dh) * J.x1 + (J.ny * dh - J.vm * dc) * J.x2;
-    f[3] = J.l1 * dq[3] + (J.nz * c2dc - J.wm * dh) * J.x1 + (J.nz * dh - J.wm * dc) * J.x2;
-    f[4] = J.l1 * dq[4] + (J.ct * c2dc - J.hm * dh) * J.x1 + (J.ct * dh - J.hm * dc) * J.x2;
-}
-
-// split Jacobian of a record acting as neighbour along d, sign s (0: npn=+1, 1: npn=-1)
-__device__ __forceinline__ Jac rec_jac(const double *R, int d, int s) {
-    Jac J;
-    J.um = R[SR_JS + 0];
-    J.vm = R[SR_JS + 1];
-    J.wm = R[SR_JS + 2];
-    J.c2 = R[SR_JS + 3];
-    J.hm = R[SR_JS + 4];
-    J.af = R[SR_JS + 5];
-    J.ct = R[SR_JD + 4 * d + 0];
-    J.nx = R[SR_JD + 4 * d + 1];
-    J.ny = R[SR_JD + 4 * d + 2];
-    J.nz = R[SR_JD + 4 * d + 3];
-    const int b = (s == 0 ? SR_JP : SR_JM) + 3 * d;
-    J.l1 = R[b + 0];
-    J.x1 = R[b + 1];
-    J.x2 = R[b + 2];
-    return J;
 }
 
 __host__ __device__ inline long long pm_size(const DevBlock &B) { return (long long)(B.ni + B.nj + B.nk - 2) * B.nj * B.nk; }
@@ -144,52 +105,23 @@ __global__ void __launch_bounds__(PREP_THREADS) k_lhs_prep(DevParams P, DevField
         srow[threadIdx.x] = valid ? 1 : 0;
         if (valid) {
             const long long id = gidx(B, i, j, k);
-            double rm = F.f[F_R][id], um = F.f[F_U][id], vm = F.f[F_V][id], wm = F.f[F_W][id], pmr = F.f[F_P][id];
-            double hint = P.g1 * pmr / rm;
-            double c2 = gama * pmr / rm;
-            double cm = sqrt(c2);
-            double v2 = um * um + vm * vm + wm * wm;
-            double hm = hint + 0.5 * v2;
-            double ae = gama - 1.0;
+            const double rm = F.f[F_R][id], um = F.f[F_U][id], vm = F.f[F_V][id], wm = F.f[F_W][id], pres = F.f[F_P][id];
+            const double hint = gama / (gama - 1.0) * pres / rm;  // gettmhmgm_ns (GasModel.f90:411-426)
             R[SR_COED] = F.f[F_COED][id];
 #pragma unroll
-            for (int m = 0; m < 5; m++) {
-                const double v = F.f[F_DQ1 + m][id];
-                R[SR_RHS + m] = v;  // store_rhs_nb (LHS.f90:1592-1613)
-            }
-            R[SR_JS + 0] = um;
-            R[SR_JS + 1] = vm;
-            R[SR_JS + 2] = wm;
-            R[SR_JS + 3] = c2;
-            R[SR_JS + 4] = hm;
-            R[SR_JS + 5] = 0.5 * ae * v2;
+            for (int m = 0; m < 5; m++) R[SR_RHS + m] = F.f[F_DQ1 + m][id];  // store_rhs_nb (LHS.f90:1592-1613)
+            R[SR_U + 0] = um;
+            R[SR_U + 1] = vm;
+            R[SR_U + 2] = wm;
+            R[SR_U + 3] = hint + 0.5 * (um * um + vm * vm + wm * wm);
+#pragma unroll
+            for (int m = 0; m < 9; m++) R[SR_G + m] = F.f[F_KCX + m][id];
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                double nx = F.f[F_KCX + 3 * d][id], ny = F.f[F_KCX + 3 * d + 1][id], nz = F.f[F_KCX + 3 * d + 2][id], nt = 0.0;
-                double rad = F.f[F_SRA + d][id];
-                double ct = nx * um + ny * vm + nz * wm + nt;
-                double cgm = fmax(sqrt(nx * nx + ny * ny + nz * nz), SML_SSS);
-                double cgm1 = 1.0 / cgm;
-                R[SR_JD + 4 * d + 0] = (ct - nt) * cgm1;
-                R[SR_JD + 4 * d + 1] = nx * cgm1;
-                R[SR_JD + 4 * d + 2] = ny * cgm1;
-                R[SR_JD + 4 * d + 3] = nz * cgm1;
-#pragma unroll
-                for (int sg = 0; sg < 2; sg++) {
-                    double dn = sg == 0 ? 1.0 : -1.0;
-                    double l1 = ct, l4 = ct + cm * cgm, l5 = ct - cm * cgm;
-                    l1 = 0.5 * (l1 + dn * rad);
-                    l4 = 0.5 * (l4 + dn * rad);
-                    l5 = 0.5 * (l5 + dn * rad);
-                    const int b = (sg == 0 ? SR_JP : SR_JM) + 3 * d;
-                    R[b + 0] = l1;
-                    R[b + 1] = (2.0 * l1 - l4 - l5) / (2.0 * c2);
-                    R[b + 2] = (l4 - l5) / (2.0 * cm);
-                }
+                const double rad = F.f[F_SRA + d][id];
+                R[SR_RAD + d] = rad;
+                R[SR_RADS + d] = P.nvis > 0 ? rad + F.f[F_SRVA + d][id] : rad;
             }
-            R[SR_SRV + 0] = F.f[F_SRVA][id];
-            R[SR_SRV + 1] = F.f[F_SRVB][id];
-            R[SR_SRV + 2] = F.f[F_SRVC][id];
             R[SR_N - 1] = 0.0;
         }
         __syncthreads();
@@ -261,11 +193,12 @@ constexpr int SWEEP_FINE_MAX_THREADS = 768;
 // shared memory of one CTA with `cpc` column slots:
 //   [SWEEP_STAGES][cpc][SR_N]  static records of a plane
 //   [SWEEP_STAGES][cpc][DYN_N] dynamic records of a plane
-//   [2 plane parity][3 dir (i,j,k)][cpc][10]  inbox from this CTA's own cells
-//   [JRING][cpc][10]           inbox from the neighbouring CTA (j direction)
+//   [2 plane parity][3 dir (i,j,k)][cpc][5]  inbox from this CTA's own cells
+//   [JRING][cpc][RING_LD]      inbox from the neighbouring CTA (j direction)
 //   mbarriers: SWEEP_STAGES (bulk copies), JRING full, JRING empty
+constexpr int RING_LD = 6;  // five terms, padded so that an entry is three 16-byte stores
 __host__ __device__ inline size_t sweep_smem_bytes(int cpc) {
-    return (size_t)SWEEP_STAGES * cpc * (SR_N + DYN_N) * 8 + (size_t)2 * 3 * cpc * 10 * 8 + (size_t)JRING * cpc * 10 * 8 +
+    return (size_t)SWEEP_STAGES * cpc * (SR_N + DYN_N) * 8 + (size_t)2 * 3 * cpc * 5 * 8 + (size_t)JRING * cpc * RING_LD * 8 +
            (size_t)(SWEEP_STAGES + 2 * JRING) * 8;
 }
 
@@ -347,10 +280,10 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
     double *sstat = smem;
     double *sdyn = sstat + (size_t)SWEEP_STAGES * cpc * SR_N;
     double *inbox = sdyn + (size_t)SWEEP_STAGES * cpc * DYN_N;
-    double *jring = inbox + (size_t)2 * 3 * cpc * 10;
-    unsigned long long *bars = (unsigned long long *)(jring + (size_t)JRING * cpc * 10);
+    double *jring = inbox + (size_t)2 * 3 * cpc * 5;
+    unsigned long long *bars = (unsigned long long *)(jring + (size_t)JRING * cpc * RING_LD);
     unsigned long long *full = bars + SWEEP_STAGES, *empty = full + JRING;
-    const size_t inbox_half = (size_t)3 * cpc * 10, inbox_dir = (size_t)cpc * 10;
+    const size_t inbox_half = (size_t)3 * cpc * 5, inbox_dir = (size_t)cpc * 5;
     const int t = threadIdx.x;
     const bool ctl = t == (int)blockDim.x - 32;  // control thread: lane 0 of the last warp
     const bool own = FINE ? (t < 16 * ncell && (t & 15) < 15) : t < 3 * ncell;
@@ -367,7 +300,7 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
     const bool has_up = qu >= 0 && qu < C, has_down = qd >= 0 && qd < C;
     const bool bconsumer = own && has_up && jj == (forward ? 0 : w - 1);
     const bool bproducer = own && d == 1 && has_down && jj == (forward ? w - 1 : 0);
-    const unsigned ring_bytes = (unsigned)nk * 80u;  // one plane of the boundary column
+    const unsigned ring_bytes = (unsigned)nk * (FINE ? 40u : 48u);  // one plane of the boundary column
     // predecessors along j and k inside the block (at the block faces the
     // reference multiplies a zero dq: ghost value or the explicit zero of
     // gs_pr_l/u, so those terms are zero); along i see `hasi` below
@@ -375,14 +308,13 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
     // destination of this thread's contribution inside the CTA
     double *dst = nullptr;
     if (own) {
-        if (d == 0) dst = inbox + (size_t)c * 10;
-        else if (d == 1 && !bproducer && (forward ? j < nj : j > 1)) dst = inbox + inbox_dir + (size_t)(c + step) * 10;
-        else if (d == 2 && (forward ? k < nk : k > 1)) dst = inbox + 2 * inbox_dir + (size_t)(c + step * w) * 10;
+        if (d == 0) dst = inbox + (size_t)c * 5;
+        else if (d == 1 && !bproducer && (forward ? j < nj : j > 1)) dst = inbox + inbox_dir + (size_t)(c + step) * 5;
+        else if (d == 2 && (forward ? k < nk : k > 1)) dst = inbox + 2 * inbox_dir + (size_t)(c + step * w) * 5;
     }
-    const double *srci = inbox + (size_t)c * 10 + m0;
-    const double *srcj = (bconsumer ? jring + (size_t)(k - 1) * 10 : inbox + inbox_dir + (size_t)c * 10) + m0;
-    const double *srck = inbox + 2 * inbox_dir + (size_t)c * 10 + m0;
-    const bool vis = lu && P.nvis > 0;
+    const double *srci = inbox + (size_t)c * 5 + m0;
+    const double *srcj = (bconsumer ? jring + (size_t)(k - 1) * RING_LD : inbox + inbox_dir + (size_t)c * 5) + m0;
+    const double *srck = inbox + 2 * inbox_dir + (size_t)c * 5 + m0;
 
     if (ctl) {
         for (int s = 0; s < SWEEP_STAGES; s++) mbar_init(&bars[s], 1);
@@ -399,7 +331,7 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
     cluster_wait();
     unsigned ring_remote = 0, full_remote = 0, empty_remote = 0;
     if (bproducer) {
-        ring_remote = remote_u32(jring + (size_t)(k - 1) * 10, qd);
+        ring_remote = remote_u32(jring + (size_t)(k - 1) * RING_LD, qd);
         full_remote = remote_u32(full, qd);
     }
     if (ctl && has_up) empty_remote = remote_u32(empty, qu);
@@ -438,7 +370,7 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
         if (gs_slot >= 0) gs_rec = M.gs[MODE == 2 ? 1 : 0] + (B.pmoff + gs_slot) * DYN_N + 5 * d + m0;
     }
     const long long gs_plane = (long long)nj * nk * DYN_N;
-    const double ae = P.gama - 1.0;
+    const double aeh = 0.5 * (P.gama - 1.0);
     for (int pi = 0; pi < nplanes; pi++) {
         const int p = pfirst + pi * step;
         const int i = p - j - k;
@@ -446,8 +378,8 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
         const bool hasi = forward ? i > 1 : i < ni;
         const int s = pi % SWEEP_STAGES;
         // the cell's coefficients (independent of this sweep's new values)
-        double coed = 0.0, base[NC], old0[NC], old1[NC], old2[NC], rv = 0.0, nn = 0.0, uu = 0.0;
-        Jac J;
+        double coed = 0.0, base[NC], old[NC], cu = 0.0, cv = 0.0, cw = 0.0, ch = 0.0, gx = 0.0, gy = 0.0, gz = 0.0, th = 0.0,
+               l = 0.0, l0 = 0.0, nn = 0.0, uu = 0.0;
         if (act) {
             const double *R = sstat + ((size_t)s * cpc + c) * SR_N;
             const double *D = sdyn + ((size_t)s * cpc + c) * DYN_N + m0;
@@ -455,16 +387,22 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
 #pragma unroll
             for (int m = 0; m < NC; m++) {
                 base[m] = MODE == 1 ? D[m] : R[SR_RHS + m0 + m];
-                // gs_pr_u: (del + dfl) + dgl of the lower neighbours, gs_pr_l: the three upper terms
-                old0[m] = MODE == 3 ? D[m] + D[5 + m] + D[10 + m] : MODE == 2 ? D[m] : 0.0;
-                old1[m] = MODE == 2 ? D[5 + m] : 0.0;
-                old2[m] = MODE == 2 ? D[10 + m] : 0.0;
+                // gs_pr_l: the upper neighbours' terms, gs_pr_u: the lower ones'
+                old[m] = MODE >= 2 ? (D[m] + D[5 + m]) + D[10 + m] : 0.0;
             }
-            J = rec_jac(R, d, forward ? 0 : 1);
-            if (vis) rv = R[SR_SRV + d];
-            if (FINE && m0 > 0) {  // row m0 of the product: (nx, um), (ny, vm), (nz, wm) or (ct, hm)
-                nn = R[SR_JD + 4 * d + (m0 & 3)];
-                uu = R[SR_JS + (m0 == 4 ? 4 : m0 - 1)];
+            cu = R[SR_U + 0];
+            cv = R[SR_U + 1];
+            cw = R[SR_U + 2];
+            ch = R[SR_U + 3];
+            gx = R[SR_G + 3 * d];
+            gy = R[SR_G + 3 * d + 1];
+            gz = R[SR_G + 3 * d + 2];
+            th = sw_theta(gx, gy, gz, cu, cv, cw);
+            l0 = sw_l<forward>(th, R[SR_RAD + d]);
+            l = lu ? sw_l<forward>(th, R[SR_RADS + d]) : l0;
+            if (FINE && m0 > 0) {  // row m0 of the terms: (gx, u), (gy, v), (gz, w) or (theta, H)
+                nn = m0 == 4 ? th : R[SR_G + 3 * d + m0 - 1];
+                uu = R[SR_U + m0 - 1];
             }
         }
         if (ctl) {
@@ -492,26 +430,11 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
         // new dq, components m0 .. m0+NC-1
         double nw[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         if (act) {
-            const double *inj = srcj + (bconsumer ? (size_t)((pi - 1) % JRING) * cpc * 10 : rd);
+            const double *inj = srcj + (bconsumer ? (size_t)((pi - 1) % JRING) * cpc * RING_LD : rd);
 #pragma unroll
             for (int m = 0; m < NC; m++) {
                 const double ci = hasi ? srci[rd + m] : 0.0, cj = hasj ? inj[m] : 0.0, ck = hask ? srck[rd + m] : 0.0;
-                if (MODE == 0 || MODE == 1) {
-                    double r0 = 1.0 * (ci + cj + ck);
-                    if (vis) {
-                        const double vi = hasi ? srci[rd + 5 + m] : 0.0, vj = hasj ? inj[5 + m] : 0.0,
-                                     vk = hask ? srck[rd + 5 + m] : 0.0;
-                        const double v = 0.5 * (vi + vj + vk);
-                        r0 = MODE == 0 ? r0 + v : r0 - v;
-                    }
-                    nw[m] = MODE == 0 ? (-base[m] + r0) * coed : base[m] - r0 * coed;
-                } else if (MODE == 2) {
-                    const double r0 = 1.0 * (ci + cj + ck - old0[m] - old1[m] - old2[m]);
-                    nw[m] = (r0 - base[m]) * coed;
-                } else {
-                    const double r0 = 1.0 * (old0[m] - ci - cj - ck);
-                    nw[m] = (r0 - base[m]) * coed;
-                }
+                nw[m] = sw_new<MODE>((ci + cj) + ck, old[m], MODE == 3 ? old[m] - base[m] : base[m], coed);
             }
         }
         const double own_nw = nw[0];  // FINE: component m0
@@ -521,51 +444,48 @@ __global__ void __launch_bounds__(FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_M
 #pragma unroll
             for (int m = 0; m < 5; m++) nw[m] = __shfl_sync(0xffffffffu, own_nw, (g + m) & 31);
         }
-        // contribution along d for the successor (rows m0 .. m0+NC-1 of mxdq_std)
-        double o[2 * NC];
+        // contribution along d for the successor (rows m0 .. m0+NC-1); og: the
+        // same without the viscous radii, the old-side term of the next sweep
+        double o[NC], og[NC];
         if (act) {
+            const double e = sw_half_dh(aeh, cu, cv, cw, nw);
             if constexpr (FINE) {
-                const double dc = J.ct * nw[0] - J.nx * nw[1] - J.ny * nw[2] - J.nz * nw[3];
-                const double dh = J.af * nw[0] - ae * (J.um * nw[1] + J.vm * nw[2] + J.wm * nw[3] - nw[4]);
-                const double c2dc = J.c2 * dc;
-                o[0] = m0 == 0 ? J.l1 * nw[0] - dh * J.x1 - dc * J.x2
-                               : J.l1 * own_nw + (nn * c2dc - uu * dh) * J.x1 + (nn * dh - uu * dc) * J.x2;
-                o[1] = rv * own_nw;
+                const double d2 = sw_half_d(gx, gy, gz, th, nw);
+                const double tm = m0 == 0 ? sw_t0(d2) : sw_tm(nn, uu, e, d2);
+                o[0] = fma(l, own_nw, tm);
+                og[0] = MODE == 1 ? fma(l0, own_nw, tm) : o[0];
             } else {
-                double f[5];
-                jac_apply(P, J, nw, f);
+                double tm[5];
+                sw_terms(gx, gy, gz, th, cu, cv, cw, ch, e, nw, tm);
 #pragma unroll
                 for (int m = 0; m < 5; m++) {
-                    o[m] = f[m];
-                    o[5 + m] = rv * nw[m];
+                    o[m] = fma(l, nw[m], tm[m]);
+                    og[m] = MODE == 1 ? fma(l0, nw[m], tm[m]) : o[m];
                 }
             }
             if (dst) {
 #pragma unroll
-                for (int m = 0; m < NC; m++) {
-                    dst[wr + m0 + m] = o[m];
-                    dst[wr + 5 + m0 + m] = o[NC + m];
-                }
+                for (int m = 0; m < NC; m++) dst[wr + m0 + m] = o[m];
             }
         } else {
 #pragma unroll
-            for (int m = 0; m < 2 * NC; m++) o[m] = 0.0;  // a boundary producer still sends the plane
+            for (int m = 0; m < NC; m++) o[m] = og[m] = 0.0;  // a boundary producer still sends the plane
         }
         if (bproducer && pi < nplanes - 1) {
             const int so = pi % JRING;
-            const unsigned a = ring_remote + (unsigned)(so * cpc * 80), mb = full_remote + (unsigned)(so * 8);
+            const unsigned a = ring_remote + (unsigned)(so * cpc * RING_LD * 8), mb = full_remote + (unsigned)(so * 8);
             if constexpr (FINE) {
                 st_async_f64(a + 8u * m0, o[0], mb);
-                st_async_f64(a + 8u * (5 + m0), o[1], mb);
             } else {
-#pragma unroll
-                for (int m = 0; m < 10; m += 2) st_async_v2(a + 8u * m, o[m], o[m + 1], mb);
+                st_async_v2(a, o[0], o[1], mb);
+                st_async_v2(a + 16u, o[2], o[3], mb);
+                st_async_v2(a + 32u, o[4], 0.0, mb);
             }
         }
         if ((MODE == 1 || MODE == 2) && act && gs_rec && (d != 0 || (forward ? i < ni : i > 1))) {
             double *G = gs_rec + (long long)(p + step - 3) * gs_plane;
 #pragma unroll
-            for (int m = 0; m < NC; m++) G[m] = o[m];
+            for (int m = 0; m < NC; m++) G[m] = og[m];
         }
         if (act && d == 0) {
             const long long pm = pmidx(B, p, j0 * nk + c);

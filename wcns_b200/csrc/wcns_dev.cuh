@@ -90,12 +90,11 @@ __host__ __device__ inline int col_slot(int j, int k, int nj, int nk, int C) {
 // static per-cell record of the sweeps (written once per step by k_lhs_prep)
 enum StatRec : int {
     SR_COED = 0, SR_RHS = 1,              // coed, rhs(5)
-    SR_JS = 6,                            // um, vm, wm, c2, hm, af
-    SR_JD = 12,                           // per direction d: ct, nx, ny, nz at SR_JD + 4d
-    SR_JP = 24,                           // npn=+1 (lower neighbour): l1, x1, x2 at SR_JP + 3d
-    SR_JM = 33,                           // npn=-1 (upper neighbour): l1, x1, x2 at SR_JM + 3d
-    SR_SRV = 42,                          // srva, srvb, srvc
-    SR_N = 46                             // record length (16-byte multiple)
+    SR_U = 6,                             // u, v, w, H
+    SR_G = 10,                            // the nine metrics, direction by direction
+    SR_RAD = 19,                          // inviscid radii
+    SR_RADS = 22,                         // inviscid plus viscous radii
+    SR_N = 26                             // record length (16-byte multiple)
 };
 constexpr int DYN_N = 16;                 // dynamic per-cell record: dq of lusgs_l, or old-side terms 5*d + m
 

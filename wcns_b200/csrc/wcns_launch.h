@@ -76,35 +76,50 @@ struct ProfMarks {
     const char **name = nullptr;
 };
 
-// Wide sweeps (k_sweep_wide.cu): a chunk of whole j-rows of one block per
-// CTA, plane-major arrays, rings of planes between neighbouring chunks.
-constexpr int WIDE_MAX_THREADS = 512;
-// 16 warps x 32 x 128 registers fill one SM's register file, four warps of
-// 4,096 registers per sub-partition
-constexpr int WIDE_MAX_REGS = 128;
-constexpr int WIDE_COEF_WORDS = 40;  // coefficient words per slot (k_sweep_wide.cu)
-struct WideChunk {
-    int blk, j0, w;         // block (0-based), first j-row (0-based) and width of the chunk
+// Wide sweeps (k_sweep_wide.cu): a block's columns in chunks of whole rows
+// (along the shorter of j and k), one or several chunks (segments) per CTA,
+// plane-major records, rings of planes between neighbouring chunks.
+// Columns per CTA: nine warps, and three helper warps, are three warps of 168
+// registers per sub-partition.
+constexpr int WIDE_THREADS = 288;
+constexpr int WIDE_PAIRS = 18;         // pairs of words per slot (k_sweep_wide.cu)
+constexpr int WIDE_SA_PAIRS = 3;       // ... of the SA model's sweeps
+constexpr int WIDE_UNITS = 10;         // 16-byte units per ring entry
+constexpr int WIDE_MAX_FOLD = 8;       // segments per CTA
+constexpr int WIDE_MIN_COLS = 32;      // columns per chunk at least (where the block has them)
+// Time of a plane without and per column of a CTA, and of a hop between CTAs,
+// microseconds (setup_sweep_wide): fitted to lusgs_l on the 65x33x17 vortex
+// (34, 51, 119 and 187 columns per CTA, 17 to 3 chunks: 84, 78, 81 and 86 us)
+// and the 64-case batch (272 columns, 2 chunks: 94 us).
+constexpr double WIDE_T0 = 0.52, WIDE_TC = 0.0013, WIDE_THOP = 1.0;
+struct WideSeg {
+    int blk, j0, w;         // block (0-based), first row (0-based) and width of the chunk
     int bnd_lo, bnd_hi;     // ring between this chunk and the previous / next one (-1: none)
-    long long pmoff;        // the block's first slot in the plane-major arrays
+    int W, cols;            // the CTA's column stride per k (thread t has row t % W, k = t / W + 1), slots per plane
+    int pmoff;              // the chunk's first slot; slot of plane s (0-based) and thread t: pmoff + s * cols + t
+};
+struct WideCta {
+    int blk, seg0, segstep, nseg;  // its chunks: segments seg0, seg0 + segstep, ...
+    int nsegmax, delay;            // segments of the block's longest CTA; planes each one runs behind the one before
+    int w;                         // width of the widest chunk
 };
 struct WideArrays {
-    long long n = 0;        // slots per word array
-    double *stat = nullptr; // WIDE_COEF_WORDS per slot: split-Jacobian coefficients, coed, srv
-    double *rhs = nullptr;  // 5
-    double *dql = nullptr;  // 5: lusgs_l's dq, the start of lusgs_u
-    double *gs1 = nullptr;  // 15: lusgs_u -> gs_pr_l, terms of the upper neighbours
-    double *gs2 = nullptr;  // 5: gs_pr_l -> gs_pr_u, summed terms of the lower neighbours
-    double *sa = nullptr;   // 6: the SA model's scalar sweeps (after wcns_sa_setup)
-    double *ring = nullptr; // [boundary][ring slot][nkmax][10]
-    unsigned *flags = nullptr;  // [boundary][produced, consumed] plane counts
-    int nbnd = 0, nkmax = 0;
+    long long n = 0;         // slots, a multiple of 32
+    double2 *rec = nullptr;  // records of 32 slots, WIDE_PAIRS pairs of words each (k_sweep_wide.cu)
+    double2 *sa = nullptr;   // the same with WIDE_SA_PAIRS, for the SA model's scalar sweeps (after wcns_sa_setup)
+    void *ring = nullptr;    // [boundary][ringn planes][nkmax * WIDE_UNITS] units of 16 bytes
+    unsigned *flags = nullptr;  // [boundary] planes read, counted on the launch's base
+    unsigned *epoch = nullptr;  // base of the ring tags
+    unsigned span = 0;          // tags of one launch
+    int nbnd = 0, nkmax = 0, ringn = 0;  // rings; longest row; planes per ring
 };
 struct WideSweep {
-    WideChunk *chunks = nullptr;  // device
-    std::vector<WideChunk> hchunks;
-    int nchunks = 0, threads = 0;
-    size_t smem_lu = 0, smem_gs = 0;
+    WideCta *ctas = nullptr;  // device
+    WideSeg *segs = nullptr;
+    std::vector<WideCta> hctas;
+    std::vector<WideSeg> hsegs;
+    int nctas = 0, threads = 0;
+    int stages[4] = {};  // planes of words in flight, per sweep
     WideArrays A;
 };
 
