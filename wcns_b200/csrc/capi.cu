@@ -345,41 +345,51 @@ static void wide_free(WcnsContext *c) {
 static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
     LaunchCtx &L = c->L;
     const int nbk = (int)c->blk.size();
-    size_t inv_smem = 0, vis_smem = 0, inv_mx_smem = 0, vis_mx_smem = 0;
+    const bool sections = c->P.nscheme == 41 || c->P.nscheme == 42;
+    size_t inv_smem = 0, vis_smem = 0, inv_mx_smem = 0, vis_mx_smem = 0, adj_smem = 0;
     for (int dir = 0; dir < 3; dir++) {
-        for (int pass = 0; pass < 4; pass++) {  // 0 inviscid, 1 viscous, 2 and 3 the same in mixed precision
+        for (int pass = 0; pass < 5; pass++) {  // 0 inviscid, 1 viscous, 2 and 3 the same in mixed precision, 4 the adjoint's operators
             std::vector<LineGroup> g;
-            int nl_max = 0, hmax = 0;
+            int hmax = 0;
             size_t sm_dir = 0;
             for (int b = 0; b < nbk; b++) {
                 const DevBlock &D = c->blk[b].d;
                 int n = dimof(D, dir);
-                if ((pass == 0 || pass == 2) && n <= NIJK2D) continue;
+                if ((pass == 0 || pass == 2 || pass == 4) && n <= NIJK2D) continue;
+                if (pass == 4 && (c->P.nvis != 0 || c->P.nscheme != 4)) continue;  // refused there
                 int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
                 int na = dimof(D, a1), nb2 = dimof(D, a2);
-                size_t per_line = pass == 0 ? rhs_invis_line_bytes(n) : pass == 1 ? rhs_vis_line_bytes(n)
-                                : pass == 2 ? rhs_invis_mx_line_bytes(n) : rhs_vis_mx_line_bytes(n);
-                // staged lines per CTA: at most 54 KB for the FP64 inviscid kernel (four
-                // 256-thread CTAs of 64 registers per SM), 108 KB for the FP64 viscous
-                // kernel (two 320-thread CTAs of 96 registers), 72 KB for the
-                // mixed-precision kernels
+                size_t per_line = pass == 0 ? rhs_invis_line_bytes(n, sections) : pass == 1 ? rhs_vis_line_bytes(n)
+                                : pass == 2 ? rhs_invis_mx_line_bytes(n) : pass == 3 ? rhs_vis_mx_line_bytes(n) : adj_line_bytes(n);
+                // staged lines per CTA: the kernel's share of the SM's shared memory for
+                // the FP64 inviscid kernel, 108 KB for the FP64 viscous kernel (two
+                // 320-thread CTAs of 96 registers), 72 KB for the mixed-precision kernels and the adjoint's
                 int NL = pass == 0 ? std::max(1, std::min({std::min(inv_cap, rhs_invis_max_lines()), 3072 / (5 * (n + 2)),
-                                                           (int)((54 * 1024) / per_line)}))
+                                                           (int)(rhs_invis_smem() / per_line)}))
                        : pass == 1 ? std::max(1, std::min({std::min(vis_cap, rhs_vis_max_lines()), 512 / (n + 1), (int)((108 * 1024) / per_line)}))
-                       : pass == 2 ? std::max(1, std::min({std::min(inv_cap, rhs_invis_mx_max_lines()), 3072 / (5 * (n + 2)),
-                                                           (int)((72 * 1024) / per_line)}))
+                       : pass == 2 || pass == 4 ? std::max(1, std::min({std::min(inv_cap, pass == 2 ? rhs_invis_mx_max_lines() : adj_max_lines()),
+                                                                        3072 / (5 * (n + 2)), (int)((72 * 1024) / per_line)}))
                                    : std::max(1, std::min({std::min(vis_cap, rhs_vis_mx_max_lines()), 512 / (n + 1), (int)((72 * 1024) / per_line)}));
-                if (pass == 1) {
-                    // the FP64 viscous kernel's heavy phase has one item per (line, half
-                    // node): of NL/2..NL lines take the count whose items fill the last
-                    // pass of the CTA's threads best, so that few threads idle at the
-                    // barrier after it (3.29 -> 3.11 ms per channel step with the larger
+                if (pass <= 1) {
+                    // the heavy phase of the FP64 kernels has one item per (line, half
+                    // node), and 13 more per end with boundary sections: of NL/2..NL
+                    // lines take the count whose items fill the last pass of the CTA's
+                    // threads best, so that few threads idle at the barrier after it
+                    // (viscous: 3.29 -> 3.11 ms per channel step with the larger
                     // staging limit)
-                    const int thr = rhs_vis_threads();
+                    const int thr = pass == 0 ? rhs_invis_threads() : rhs_vis_threads();
+                    int per = n + 1;
+                    if (pass == 0 && sections)
+                        for (int lr = -1; lr <= 1; lr += 2)
+                            for (const HReg &R : c->blk[b].regs)
+                                if ((R.bctype == 4 || R.bctype == 2) && R.s_nd == dir + 1 && R.s_lr == lr) {
+                                    per += 13;
+                                    break;
+                                }
                     int best = NL;
                     double best_fill = 0.0;
                     for (int q = NL; q >= std::max(1, (NL + 1) / 2); q--) {
-                        const int items = q * (n + 1), rounds = (items + thr - 1) / thr;
+                        const int items = q * per, rounds = (items + thr - 1) / thr;
                         const double fill = (double)items / ((double)rounds * thr);
                         if (fill > best_fill + 1e-9) {
                             best_fill = fill;
@@ -392,14 +402,12 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
                     for (int a = 1; a <= na; a += NL) {
                         LineGroup lg{b, a, bb, std::min(NL, na - a + 1)};
                         g.push_back(lg);
-                        nl_max = std::max(nl_max, lg.nl);
                         sm_dir = std::max(sm_dir, per_line * lg.nl);
                     }
                 hmax = std::max(hmax, n + 1);
             }
-            DirTable &T = pass == 0 ? L.inv[dir] : pass == 1 ? L.vis[dir] : pass == 2 ? L.inv_mx[dir] : L.vis_mx[dir];
+            DirTable &T = pass == 0 ? L.inv[dir] : pass == 1 ? L.vis[dir] : pass == 2 ? L.inv_mx[dir] : pass == 3 ? L.vis_mx[dir] : L.adj[dir];
             T.ngroups = (int)g.size();
-            T.nl_max = nl_max;
             T.hmax = hmax;
             T.smem = sm_dir;
             if (T.groups) {  // a rebuild (wcns_set_shape): the old table goes
@@ -408,12 +416,12 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
             }
             T.groups = c->up(g);
             size_t sm = sm_dir;
-            size_t &acc = pass == 0 ? inv_smem : pass == 1 ? vis_smem : pass == 2 ? inv_mx_smem : vis_mx_smem;
+            size_t &acc = pass == 0 ? inv_smem : pass == 1 ? vis_smem : pass == 2 ? inv_mx_smem : pass == 3 ? vis_mx_smem : adj_smem;
             acc = std::max(acc, sm);
         }
     }
     if (inv_smem > 227 * 1024 || vis_smem > 227 * 1024) { set_err("line too long for shared memory"); return WCNS_ERR_ARGUMENT; }
-    setup_rhs_invis_attrs(std::max<size_t>(inv_smem, 48 * 1024));
+    setup_rhs_invis_attrs(std::max<size_t>(inv_smem, 48 * 1024), c->P.nflux);
     setup_rhs_vis_attrs(std::max<size_t>(vis_smem, 48 * 1024));
     if (inv_mx_smem > 227 * 1024 || vis_mx_smem > 227 * 1024) { set_err("line too long for shared memory"); return WCNS_ERR_ARGUMENT; }
     setup_rhs_mx_attrs(std::max<size_t>(inv_mx_smem, 48 * 1024), std::max<size_t>(vis_mx_smem, 48 * 1024));

@@ -748,17 +748,14 @@ __global__ void k_adj_reduce(const DevBlock *__restrict__ blocks, double *y, con
 // ---------------------------------------------------------------------------
 // launches
 // ---------------------------------------------------------------------------
-static size_t adj_smem(const LaunchCtx &c, int dir) {
-    int nmax = 0;
-    for (int b = 0; b < c.nblocks; b++) nmax = std::max(nmax, dimof(c.hblocks[b], dir));
-    return (size_t)c.inv[dir].nl_max * adj_line_stride(nmax) * sizeof(double);
-}
+size_t adj_line_bytes(int n) { return (size_t)adj_line_stride(n) * sizeof(double); }
+int adj_max_lines() { return INV_LINES_DEFAULT; }
 
 void launch_rhs_invis_jvp(const LaunchCtx &c, const double *v, double *out) {
     for (int d = 0; d < 3; d++) {
-        const DirTable &T = c.inv[d];
+        const DirTable &T = c.adj[d];
         if (!T.ngroups) continue;
-        const size_t sm = adj_smem(c, d);
+        const size_t sm = T.smem;
         if (d == 0) {
             cudaFuncSetAttribute(k_rhs_invis_jvp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_rhs_invis_jvp<0><<<T.ngroups, 256, sm, c.stream>>>(*c.P, *c.F, c.blocks, T.groups, v, out, c.total);
@@ -774,9 +771,9 @@ void launch_rhs_invis_jvp(const LaunchCtx &c, const double *v, double *out) {
 
 void launch_rhs_invis_vjp(const LaunchCtx &c, const double *lam, double *out, bool fold) {
     for (int d = 0; d < 3; d++) {
-        const DirTable &T = c.inv[d];
+        const DirTable &T = c.adj[d];
         if (!T.ngroups) continue;
-        const size_t sm = adj_smem(c, d);
+        const size_t sm = T.smem;
         if (d == 0) {
             cudaFuncSetAttribute(k_rhs_invis_vjp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_rhs_invis_vjp<0><<<T.ngroups, 256, sm, c.stream>>>(*c.P, *c.F, c.blocks, T.groups, lam, out, c.total);

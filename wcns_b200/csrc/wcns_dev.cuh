@@ -293,143 +293,106 @@ __device__ __forceinline__ int flux_vl_pn(const DevParams &P, const double *prim
     return bad;
 }
 
-// flux (Convect.f90:1245-1272) with getem (GasModel.f90:358-374)
-__device__ __forceinline__ void phys_flux(double gama, const double *prim, double nx, double ny, double nz, double nt,
-                                          double *f) {
-    double rm = prim[0], um = prim[1], vm = prim[2], wm = prim[3], pm = prim[4];
-    double em = pm / (gama - 1.0) + 0.5 * rm * (um * um + vm * vm + wm * wm);
-    double cit = nx * um + ny * vm + nz * wm + nt;
-    f[0] = rm * cit;
-    f[1] = f[0] * um + nx * pm;
-    f[2] = f[0] * vm + ny * pm;
-    f[3] = f[0] * wm + nz * pm;
-    f[4] = (em + pm) * cit - pm * nt;
+// a / b from r = 1 / b: the quotient of the two rounded values corrected by
+// its remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990), the rounded quotient but for cases rarer than
+// one in 1e12.  For b and 1 / b finite and normal; a division costs a dozen
+// instructions and a branch, this three.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+    const double q = a * r;
+    return fma(fma(-q, b, a), r, q);
 }
 
-// flux_Roe (flux.f90:116-244).  Returns 1 when c^2 <= 0.
-__device__ __forceinline__ int flux_roe(const DevParams &P, const double *qlin, const double *qrin, double nx,
-                                        double ny, double nz, double nt, double *f) {
-    const double gama = P.gama;
-    double ql[5], qr[5], fl[5], fr[5], dq[5];
+// 1 / b and 1 / sqrt(x) of normal numbers from the hardware's approximation
+// (relative error below 2^-20) by one step of the iteration of third order
+// (Householder), to within an ulp or two: where the last bit does not matter.
+__device__ __forceinline__ double recip(double b) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    const double e = fma(-b, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ double recip_sqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+
+// flux_Roe (flux.f90:116-244) for the FP64 residual: the central part with the
+// operations of the reference and in their order; what the jump multiplies with
+// short reciprocals and roots, and sqrt(rl rr) as rl sqrt(rr / rl).
+// gama1_1 = 1 / (gama - 1); same: ql equals qr, which leaves the central part.
+// Returns 1 when c^2 <= 0.
+__device__ __forceinline__ int flux_roe(const DevParams &P, double gama1_1, const double *ql, const double *qr, double nx,
+                                             double ny, double nz, double nt, bool same, double *f) {
+    const double gama = P.gama, gama1 = gama - 1.0, gama2 = gama / gama1;
+    const double v2l = ql[1] * ql[1] + ql[2] * ql[2] + ql[3] * ql[3], v2r = qr[1] * qr[1] + qr[2] * qr[2] + qr[3] * qr[3];
+    double s[5];  // fr + fl
+    {
+        // flux (Convect.f90:1245-1272) with getem (GasModel.f90:358-374)
+        const double el = div_by(ql[4], gama1, gama1_1) + 0.5 * ql[0] * v2l, er = div_by(qr[4], gama1, gama1_1) + 0.5 * qr[0] * v2r;
+        const double cl = nx * ql[1] + ny * ql[2] + nz * ql[3] + nt, cr = nx * qr[1] + ny * qr[2] + nz * qr[3] + nt;
+        const double ml = ql[0] * cl, mr = qr[0] * cr;
+        s[0] = mr + ml;
+        s[1] = (mr * qr[1] + nx * qr[4]) + (ml * ql[1] + nx * ql[4]);
+        s[2] = (mr * qr[2] + ny * qr[4]) + (ml * ql[2] + ny * ql[4]);
+        s[3] = (mr * qr[3] + nz * qr[4]) + (ml * ql[3] + nz * ql[4]);
+        s[4] = ((er + qr[4]) * cr - qr[4] * nt) + ((el + ql[4]) * cl - ql[4] * nt);
+    }
+    if (same) {
 #pragma unroll
-    for (int m = 0; m < 5; m++) { ql[m] = qlin[m]; qr[m] = qrin[m]; }
-    phys_flux(gama, ql, nx, ny, nz, nt, fl);
-    phys_flux(gama, qr, nx, ny, nz, nt, fr);
-#pragma unroll
-    for (int m = 0; m < 5; m++) dq[m] = qr[m] - ql[m];
-    double gama1 = gama - 1.0;
-    double gama2 = gama / gama1;
-    ql[4] = gama2 * ql[4] / ql[0] + 0.5 * (ql[1] * ql[1] + ql[2] * ql[2] + ql[3] * ql[3]);
-    qr[4] = gama2 * qr[4] / qr[0] + 0.5 * (qr[1] * qr[1] + qr[2] * qr[2] + qr[3] * qr[3]);
-    double qroe0 = sqrt(ql[0] * qr[0]);
-    double rrl = sqrt(qr[0] / ql[0]);
-    double rrl_1 = rrl + 1.0;
-    double um = (ql[1] + qr[1] * rrl) / rrl_1;
-    double vm = (ql[2] + qr[2] * rrl) / rrl_1;
-    double wm = (ql[3] + qr[3] * rrl) / rrl_1;
-    double hm = (ql[4] + qr[4] * rrl) / rrl_1;
-    double rm = qroe0;
-    double c2 = (hm - 0.5 * (um * um + vm * vm + wm * wm)) * gama1;
-    int bad = c2 <= 0.0 ? 1 : 0;
-    double c = sqrt(c2);
-    double cta = um * nx + vm * ny + wm * nz + nt;
-    double cgm = fmax(sqrt(nx * nx + ny * ny + nz * nz), SML_SSS);
-    double cgm1 = 1.0 / cgm;
+        for (int m = 0; m < 5; m++) f[m] = 0.5 * s[m];
+        return ql[4] / ql[0] <= 0.0 ? 1 : 0;
+    }
+    const double rl1 = recip(ql[0]);
+    const double hl = fma(gama2, ql[4] * rl1, 0.5 * v2l), hr = fma(gama2, qr[4] * recip(qr[0]), 0.5 * v2r);
+    const double rr = qr[0] * rl1, rrl = rr * recip_sqrt(rr), w = recip(rrl + 1.0), rm = ql[0] * rrl;
+    const double um = fma(qr[1], rrl, ql[1]) * w, vm = fma(qr[2], rrl, ql[2]) * w, wm = fma(qr[3], rrl, ql[3]) * w,
+                 hm = fma(hr, rrl, hl) * w;
+    const double c2 = (hm - 0.5 * fma(um, um, fma(vm, vm, wm * wm))) * gama1;
+    const int bad = c2 <= 0.0 ? 1 : 0;
+    const double c_1 = recip_sqrt(c2), c = c2 * c_1;
+    const double cta = fma(um, nx, fma(vm, ny, wm * nz)) + nt;
+    const double k2 = fmax(fma(nx, nx, fma(ny, ny, nz * nz)), SML_SSS * SML_SSS), cgm1 = recip_sqrt(k2), cgm = k2 * cgm1;
     nx = nx * cgm1;
     ny = ny * cgm1;
     nz = nz * cgm1;
-    double ccgm = c * cgm;
-    double l1 = fabs(cta - ccgm), l4 = fabs(cta), l5 = fabs(cta + ccgm);
-    double l12 = l1 * l1, l42 = l4 * l4, l52 = l5 * l5;
-    double deti = P.efix * cgm;
-    double det2 = deti * deti;
-    l1 = sqrt(l12 + det2);
-    l4 = sqrt(l42 + det2);
-    l5 = sqrt(l52 + det2);
-    double dcta = dq[1] * nx + dq[2] * ny + dq[3] * nz;
-    double cta1 = cta * cgm1;
-    double rodcta = qroe0 * dcta;
-    double dp_c2 = dq[4] / c2;
-    double rodctac = rodcta / c;
-    double a1 = l4 * (dq[0] - dp_c2);
-    double a2 = l5 * (dp_c2 + rodctac) * 0.5;
-    double a3 = l1 * (dp_c2 - rodctac) * 0.5;
-    double a4 = a1 + a2 + a3;
-    double a5 = c * (a2 - a3);
-    double a6 = l4 * (rm * dq[1] - nx * rodcta);
-    double a7 = l4 * (rm * dq[2] - ny * rodcta);
-    double a8 = l4 * (rm * dq[3] - nz * rodcta);
-    double df0 = a4;
-    double df1 = um * a4 + nx * a5 + a6;
-    double df2 = vm * a4 + ny * a5 + a7;
-    double df3 = wm * a4 + nz * a5 + a8;
-    double df4 = hm * a4 + cta1 * a5 + um * a6 + vm * a7 + wm * a8 - c2 * a1 / gama1;
-    f[0] = 0.5 * (fr[0] + fl[0] - df0);
-    f[1] = 0.5 * (fr[1] + fl[1] - df1);
-    f[2] = 0.5 * (fr[2] + fl[2] - df2);
-    f[3] = 0.5 * (fr[3] + fl[3] - df3);
-    f[4] = 0.5 * (fr[4] + fl[4] - df4);
+    const double ccgm = c * cgm, deti = P.efix * cgm, det2 = deti * deti, lm = cta - ccgm, lp = cta + ccgm;
+    // the floor stands for a zero root (no entropy fix and a zero eigenvalue)
+    auto root = [](double x) { x = fmax(x, 1.0e-290); return x * recip_sqrt(x); };
+    const double l1 = root(fma(lm, lm, det2)), l4 = root(fma(cta, cta, det2)), l5 = root(fma(lp, lp, det2));
+    const double d0 = qr[0] - ql[0], d1 = qr[1] - ql[1], d2 = qr[2] - ql[2], d3 = qr[3] - ql[3], d4 = qr[4] - ql[4];
+    const double rodcta = rm * fma(d1, nx, fma(d2, ny, d3 * nz));
+    const double dp_c2 = d4 * c_1 * c_1, rodctac = rodcta * c_1;
+    const double a1 = l4 * (d0 - dp_c2), a2 = 0.5 * l5 * (dp_c2 + rodctac), a3 = 0.5 * l1 * (dp_c2 - rodctac);
+    const double a4 = a1 + a2 + a3, a5 = c * (a2 - a3);
+    const double a6 = l4 * fma(rm, d1, -nx * rodcta), a7 = l4 * fma(rm, d2, -ny * rodcta), a8 = l4 * fma(rm, d3, -nz * rodcta);
+    f[0] = 0.5 * (s[0] - a4);
+    f[1] = 0.5 * (s[1] - fma(um, a4, fma(nx, a5, a6)));
+    f[2] = 0.5 * (s[2] - fma(vm, a4, fma(ny, a5, a7)));
+    f[3] = 0.5 * (s[3] - fma(wm, a4, fma(nz, a5, a8)));
+    f[4] = 0.5 * (s[4] - (fma(hm, a4, cta * cgm1 * a5) + fma(um, a6, fma(vm, a7, wm * a8)) - c2 * a1 * gama1_1));
     return bad;
 }
 
-// the flux routine chosen by nflux (Convect.f90:12-46): 1 Steger-Warming,
-// 2 Van Leer, 3 Roe.  Returns the number of c^2 failures.
-__device__ __forceinline__ int flux_type(const DevParams &P, const double *ql, const double *qr, double nx, double ny,
-                                         double nz, double nt, double *f) {
-    if (P.nflux == 2) {
-        double fl[5], fr[5];
-        int bad = flux_vl_pn(P, ql, nx, ny, nz, nt, fl, 1);
+// the flux-vector splittings chosen by nflux (Convect.f90:12-46): 1
+// Steger-Warming, 2 Van Leer.  Returns the number of c^2 failures.
+template <int NFLUX>
+__device__ __forceinline__ int flux_split(const DevParams &P, const double *ql, const double *qr, double nx, double ny, double nz,
+                                          double nt, double *f) {
+    double fl[5], fr[5];
+    int bad = 0;
+    if (NFLUX == 2) {
+        bad = flux_vl_pn(P, ql, nx, ny, nz, nt, fl, 1);
         bad += flux_vl_pn(P, qr, nx, ny, nz, nt, fr, -1);
-#pragma unroll
-        for (int m = 0; m < 5; m++) f[m] = fl[m] + fr[m];
-        return bad;
-    }
-    if (P.nflux == 1) {
-        double fl[5], fr[5];
+    } else {
         flux_sw_pn(P, ql, nx, ny, nz, nt, fl, 1);
         flux_sw_pn(P, qr, nx, ny, nz, nt, fr, -1);
-#pragma unroll
-        for (int m = 0; m < 5; m++) f[m] = fl[m] + fr[m];
-        return 0;
     }
-    return flux_roe(P, ql, qr, nx, ny, nz, nt, f);
-}
-
-// mxdq_std (LHS.f90:756-828) with gettmhmgm_ns (GasModel.f90:411-426)
-__device__ __forceinline__ void mxdq_std(const DevParams &P, const double *prim, double gx, double gy, double gz,
-                                         const double *dq, double *f, double rad, int npn) {
-    const double gama = P.gama;
-    double rm = prim[0], um = prim[1], vm = prim[2], wm = prim[3], pm = prim[4];
-    double hint = P.g1 * pm / rm;
-    double c2 = gama * pm / rm;
-    double cm = sqrt(c2);
-    double v2 = um * um + vm * vm + wm * wm;
-    double hm = hint + 0.5 * v2;
-    double nx = gx, ny = gy, nz = gz, nt = 0.0;
-    double ct = nx * um + ny * vm + nz * wm + nt;
-    double cgm = fmax(sqrt(nx * nx + ny * ny + nz * nz), SML_SSS);
-    double dn = (double)npn;
-    double l1 = ct, l4 = ct + cm * cgm, l5 = ct - cm * cgm;
-    l1 = 0.5 * (l1 + dn * rad);
-    l4 = 0.5 * (l4 + dn * rad);
-    l5 = 0.5 * (l5 + dn * rad);
-    double x1 = (2.0 * l1 - l4 - l5) / (2.0 * c2);
-    double x2 = (l4 - l5) / (2.0 * cm);
-    double cgm1 = 1.0 / cgm;
-    nx = nx * cgm1;
-    ny = ny * cgm1;
-    nz = nz * cgm1;
-    ct = (ct - nt) * cgm1;
-    double ae = gama - 1.0;
-    double af = 0.5 * ae * v2;
-    double dc = ct * dq[0] - nx * dq[1] - ny * dq[2] - nz * dq[3];
-    double dh = af * dq[0] - ae * (um * dq[1] + vm * dq[2] + wm * dq[3] - dq[4]);
-    double c2dc = c2 * dc;
-    f[0] = l1 * dq[0] - dh * x1 - dc * x2;
-    f[1] = l1 * dq[1] + (nx * c2dc - um * dh) * x1 + (nx * dh - um * dc) * x2;
-    f[2] = l1 * dq[2] + (ny * c2dc - vm * dh) * x1 + (ny * dh - vm * dc) * x2;
-    f[3] = l1 * dq[3] + (nz * c2dc - wm * dh) * x1 + (nz * dh - wm * dc) * x2;
-    f[4] = l1 * dq[4] + (ct * c2dc - hm * dh) * x1 + (ct * dh - hm * dc) * x2;
+#pragma unroll
+    for (int m = 0; m < 5; m++) f[m] = fl[m] + fr[m];
+    return bad;
 }
 
 // Sutherland viscosity, compute_visl_ns (GasModel.f90:219-235)

@@ -15,7 +15,7 @@ struct LineGroup {
 
 struct DirTable {
     LineGroup *groups = nullptr;  // device
-    int ngroups = 0, nl_max = 0, hmax = 0;
+    int ngroups = 0, hmax = 0;
     size_t smem = 0;              // dynamic shared memory of the launch (max over groups)
 };
 
@@ -139,6 +139,7 @@ struct LaunchCtx {
     int nblocks = 0;
     int *err = nullptr;            // device error slots
     DirTable inv[3], vis[3];
+    DirTable adj[3];  // lines of the adjoint's inviscid operators
     // mixed precision (wcns_set_precision(ctx, 32)): the residual kernels of
     // k_rhs_mixed.cu with their own line groups, and FP32 node derivatives
     // of (u,v,w,T) in the storage of the FP64 ones (12 x total floats)
@@ -233,8 +234,10 @@ inline void launch_block_clusters(void (*kern)(KArgs...), int nblocks, int threa
 }
 
 void launch_rhs_invis(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
-void setup_rhs_invis_attrs(size_t max_smem);
-size_t rhs_invis_line_bytes(int n);  // shared memory of one line in k_rhs_invis
+void setup_rhs_invis_attrs(size_t max_smem, int nflux);
+size_t rhs_invis_line_bytes(int n, bool sections);  // shared memory of one line in k_rhs_invis
+int rhs_invis_threads();             // threads per CTA in k_rhs_invis
+size_t rhs_invis_smem();             // staged lines per CTA at most, bytes
 int rhs_invis_max_lines();           // lines per CTA in k_rhs_invis
 void launch_node_derivatives(const LaunchCtx &c);
 void launch_rhs_vis(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
@@ -244,6 +247,8 @@ void setup_rhs_vis_attrs(size_t max_smem);
 size_t rhs_vis_line_bytes(int n);  // shared memory of one line in k_rhs_vis
 int rhs_vis_max_lines();           // lines per CTA in k_rhs_vis
 int rhs_vis_threads();            // threads per CTA in k_rhs_vis
+size_t adj_line_bytes(int n);     // shared memory of one line in the adjoint's kernels
+int adj_max_lines();              // lines per CTA in the adjoint's kernels
 // mixed-precision residual (k_rhs_mixed.cu)
 void launch_rhs_invis_mx(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
 void launch_rhs_vis_mx(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
