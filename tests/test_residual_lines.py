@@ -45,3 +45,17 @@ def test_inviscid_lines(dims, nscheme, nflux):
     g.r_h_s_invis(); o.phase("rhs_invis")
     errs = compare_fields(g, o, DQ)
     assert max(errs.values()) <= 1e-12, errs
+
+
+@pytest.mark.parametrize("dims", DIMS + [(4, 6, 7), (9, 5, 3), (6, 4, 5)], ids=lambda d: "x".join(map(str, d)))
+def test_viscous_lines(dims):
+    from oracle.pyoracle import Oracle
+    from wcns_b200.solver import Wcns
+    case = _case(dims, 4, 1)
+    case.params.nvis = 1
+    g, o = Wcns(case), Oracle(case)
+    g.boundary_all(); o.phase("boundary_all")
+    g.initial_q_dq_c_t(); o.phase("initial_q_dq_c_t")
+    g.r_h_s_vis(); o.phase("rhs_vis")
+    errs = compare_fields(g, o, DQ)
+    assert max(errs.values()) <= 1e-12, errs

@@ -341,7 +341,10 @@ static void wide_free(WcnsContext *c) {
 
 // Line groups of the residual kernels for every direction (passes 2 and 3:
 // the mixed-precision kernels): at most inv_cap / vis_cap lines of a block
-// per CTA, fewer where the staged lines would pass 72 KB of shared memory.
+// per CTA, fewer where the staged lines would pass the kernel's share of shared
+// memory.  Longer lines than MAX_LINE are refused, as ever: nothing is tested there.
+constexpr int MAX_LINE = 997;
+
 static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
     LaunchCtx &L = c->L;
     const int nbk = (int)c->blk.size();
@@ -350,36 +353,38 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
     for (int dir = 0; dir < 3; dir++) {
         for (int pass = 0; pass < 5; pass++) {  // 0 inviscid, 1 viscous, 2 and 3 the same in mixed precision, 4 the adjoint's operators
             std::vector<LineGroup> g;
-            int hmax = 0;
             size_t sm_dir = 0;
             for (int b = 0; b < nbk; b++) {
                 const DevBlock &D = c->blk[b].d;
                 int n = dimof(D, dir);
                 if ((pass == 0 || pass == 2 || pass == 4) && n <= NIJK2D) continue;
+                if (n > MAX_LINE) { set_err("line too long for shared memory"); return WCNS_ERR_ARGUMENT; }
                 if (pass == 4 && (c->P.nvis != 0 || c->P.nscheme != 4)) continue;  // refused there
                 int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
                 int na = dimof(D, a1), nb2 = dimof(D, a2);
-                size_t per_line = pass == 0 ? rhs_invis_line_bytes(n, sections) : pass == 1 ? rhs_vis_line_bytes(n)
+                size_t per_line = pass == 0 ? rhs_invis_line_bytes(n, sections) : pass == 1 ? rhs_vis_line_bytes(dir, n, 1)
                                 : pass == 2 ? rhs_invis_mx_line_bytes(n) : pass == 3 ? rhs_vis_mx_line_bytes(n) : adj_line_bytes(n);
                 // staged lines per CTA: the kernel's share of the SM's shared memory for
-                // the FP64 inviscid kernel, 108 KB for the FP64 viscous kernel (two
-                // 320-thread CTAs of 96 registers), 72 KB for the mixed-precision kernels and the adjoint's
+                // the FP64 inviscid kernel, 72 KB for the mixed-precision kernels and the
+                // adjoint's; the FP64 viscous kernel takes as many as its threads
                 int NL = pass == 0 ? std::max(1, std::min({std::min(inv_cap, rhs_invis_max_lines()), 3072 / (5 * (n + 2)),
                                                            (int)(rhs_invis_smem() / per_line)}))
-                       : pass == 1 ? std::max(1, std::min({std::min(vis_cap, rhs_vis_max_lines()), 512 / (n + 1), (int)((108 * 1024) / per_line)}))
+                       : pass == 1 ? std::max(1, std::min(vis_cap, rhs_vis_lines(n)))
                        : pass == 2 || pass == 4 ? std::max(1, std::min({std::min(inv_cap, pass == 2 ? rhs_invis_mx_max_lines() : adj_max_lines()),
                                                                         3072 / (5 * (n + 2)), (int)((72 * 1024) / per_line)}))
                                    : std::max(1, std::min({std::min(vis_cap, rhs_vis_mx_max_lines()), 512 / (n + 1), (int)((72 * 1024) / per_line)}));
-                if (pass <= 1) {
-                    // the heavy phase of the FP64 kernels has one item per (line, half
-                    // node), and 13 more per end with boundary sections: of NL/2..NL
-                    // lines take the count whose items fill the last pass of the CTA's
-                    // threads best, so that few threads idle at the barrier after it
-                    // (viscous: 3.29 -> 3.11 ms per channel step with the larger
-                    // staging limit)
-                    const int thr = pass == 0 ? rhs_invis_threads() : rhs_vis_threads();
+                if (pass == 1) {  // rows of equal share
+                    const int ng = (na + NL - 1) / NL;
+                    NL = (na + ng - 1) / ng;
+                }
+                if (pass == 0) {
+                    // the heavy phase has one item per (line, half node), and 13 more
+                    // per end with boundary sections: of NL/2..NL lines take the count
+                    // whose items fill the last pass of the CTA's threads best, so that
+                    // few threads idle at the barrier after it
+                    const int thr = rhs_invis_threads();
                     int per = n + 1;
-                    if (pass == 0 && sections)
+                    if (sections)
                         for (int lr = -1; lr <= 1; lr += 2)
                             for (const HReg &R : c->blk[b].regs)
                                 if ((R.bctype == 4 || R.bctype == 2) && R.s_nd == dir + 1 && R.s_lr == lr) {
@@ -402,13 +407,11 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
                     for (int a = 1; a <= na; a += NL) {
                         LineGroup lg{b, a, bb, std::min(NL, na - a + 1)};
                         g.push_back(lg);
-                        sm_dir = std::max(sm_dir, per_line * lg.nl);
+                        sm_dir = std::max(sm_dir, pass == 1 ? rhs_vis_line_bytes(dir, n, lg.nl) : per_line * lg.nl);
                     }
-                hmax = std::max(hmax, n + 1);
             }
             DirTable &T = pass == 0 ? L.inv[dir] : pass == 1 ? L.vis[dir] : pass == 2 ? L.inv_mx[dir] : pass == 3 ? L.vis_mx[dir] : L.adj[dir];
             T.ngroups = (int)g.size();
-            T.hmax = hmax;
             T.smem = sm_dir;
             if (T.groups) {  // a rebuild (wcns_set_shape): the old table goes
                 c->owned.erase(std::remove(c->owned.begin(), c->owned.end(), (void *)T.groups), c->owned.end());

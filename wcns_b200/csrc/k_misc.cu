@@ -327,6 +327,7 @@ __global__ void k_combine_dq(DevFields F, const DevBlock *__restrict__ blocks, c
         const long long id = gidx(B, i, j, k);
 #pragma unroll
         for (int m = 0; m < 5; m++) {
+            if (sub && m == 0) continue;  // no viscous mass flux
             double v = F.f[F_DQ1 + m][id];
             if (c1) v = sub ? v - c1[m * stride + id] : v + c1[m * stride + id];
             if (c2) v = sub ? v - c2[m * stride + id] : v + c2[m * stride + id];

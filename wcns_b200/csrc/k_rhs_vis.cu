@@ -14,15 +14,22 @@
 //   * per point: FLUX_DXYZ and dq -= re*dFv.
 // The boundary flag of a line is the reference's uvwt(4,-2) test: -1 when the
 // third ghost density is negative, otherwise the ghost temperature.
+#include <algorithm>
+
 #include "wcns_dev.cuh"
 #include "wcns_launch.h"
 
 namespace wcns {
 
 // ---------------------------------------------------------------------------
-// node derivatives: one thread per interior point
+// node derivatives and the molecular viscosity: one thread per interior point
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256, 4) k_node_deriv(DevParams P, DevFields F, const DevBlock *__restrict__ blocks, int nblocks) {
+// Bound by the instructions around its 48 loads: fields are indexed with 32 bits
+// (a field has far fewer points than that: HBM would hold 4e8), and the one-sided
+// formulas run only where an end has a boundary, not wherever a line ends.
+// The viscosity goes to memory here, so that the three line kernels read 8 bytes
+// where each would evaluate a root and a division per point.
+__global__ void __launch_bounds__(256, 5) k_node_deriv(DevParams P, DevFields F, const DevBlock *__restrict__ blocks, int nblocks) {
     int bi = blockIdx.y;
     if (bi >= nblocks) return;
     const DevBlock B = blocks[bi];
@@ -30,33 +37,56 @@ __global__ void __launch_bounds__(256, 4) k_node_deriv(DevParams P, DevFields F,
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         decode_point(B, p, i, j, k);
-        long long id = gidx(B, i, j, k);
+        const int id = (int)gidx(B, i, j, k);
+        // viscosities at the point, as the reference's visl/vist arrays:
+        // mu + vist and mu*cp_prl + vist*cp_prt (vist = 0 when laminar)
+        const double mu = sutherland(P, __ldg(F.f[F_T] + id));
+        const double vt = F.f[F_VIST] ? __ldg(F.f[F_VIST] + id) : 0.0;
+        F.f[F_MU][id] = mu + vt;
+        F.f[F_MU + 1][id] = mu * B.cp_prl + vt * B.cp_prt;
+#pragma unroll 1
         for (int d = 0; d < 3; d++) {
-            int n = dimof(B, d);
-            int l = d == 0 ? i : (d == 1 ? j : k);
-            long long st = dstride(B, d);
-            long long l0 = id - (long long)l * st;  // index of position 0 on the line
-            double rl = __ldg(F.f[F_R] + l0 - 2 * st), rr = __ldg(F.f[F_R] + l0 + (long long)(n + 3) * st);
-            bool fl = rl < 0.0 ? true : (__ldg(F.f[F_T] + l0 - 2 * st) < 0.0);
-            bool fr = rr < 0.0 ? true : (__ldg(F.f[F_T] + l0 + (long long)(n + 3) * st) < 0.0);
-            for (int m = 0; m < 4; m++) {
-                const double *u = F.f[m == 3 ? F_T : F_U + m] + l0;
-                auto U = [&](int x) { return __ldg(u + (long long)x * st); };
-                double du;
-                if (n <= NIJK2ND) {
-                    du = 0.5 * (U(l + 1) - U(l - 1));
-                } else if (fl && l == 1) {
-                    du = (-11. * U(1) + 18. * U(2) - 9. * U(3) + 2. * U(4)) / 6.0;
-                } else if (fl && l == 2) {
-                    du = (-3.0 * U(1) + -10.0 * U(2) + 18.0 * U(3) + -6.0 * U(4) + 1.0 * U(5)) / 12.0;
-                } else if (fr && l == n) {
-                    du = -(-11. * U(n) + 18. * U(n - 1) - 9.0 * U(n - 2) + 2. * U(n - 3)) / 6.0;
-                } else if (fr && l == n - 1) {
-                    du = -(-3.0 * U(n) + -10.0 * U(n - 1) + 18.0 * U(n - 2) + -6.0 * U(n - 3) + 1.0 * U(n - 4)) / 12.0;
-                } else {
-                    du = (8.0 * (U(l + 1) - U(l - 1)) + -1.0 * (U(l + 2) - U(l - 2))) / 12.0;
+            const int n = dimof(B, d);
+            const int l = d == 0 ? i : (d == 1 ? j : k);
+            const int st = (int)dstride(B, d);
+            bool fl = false, fr = false;
+            const int l0 = id - l * st;  // index of position 0 on the line
+            if (n > NIJK2ND) {
+                if (l <= 2) fl = __ldg(F.f[F_R] + l0 - 2 * st) < 0.0 ? true : (__ldg(F.f[F_T] + l0 - 2 * st) < 0.0);
+                else if (l >= n - 1) fr = __ldg(F.f[F_R] + l0 + (n + 3) * st) < 0.0 ? true : (__ldg(F.f[F_T] + l0 + (n + 3) * st) < 0.0);
+            }
+            if (n <= NIJK2ND) {
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    const double *u = F.f[m == 3 ? F_T : F_U + m] + id;
+                    F.f[F_DUV0 + m + 4 * d][id] = 0.5 * (__ldg(u + st) - __ldg(u - st));
                 }
-                F.f[F_DUV0 + m + 4 * d][id] = du;
+            } else if (!fl && !fr) {  // the interior formula
+                double v[4][4];
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    const double *u = F.f[m == 3 ? F_T : F_U + m] + id;
+                    v[m][0] = __ldg(u - 2 * st);
+                    v[m][1] = __ldg(u - st);
+                    v[m][2] = __ldg(u + st);
+                    v[m][3] = __ldg(u + 2 * st);
+                }
+#pragma unroll
+                for (int m = 0; m < 4; m++)
+                    F.f[F_DUV0 + m + 4 * d][id] = div_by(8.0 * (v[m][2] - v[m][1]) + -1.0 * (v[m][3] - v[m][0]), 12.0, 1.0 / 12.0);
+            } else {  // one-sided at the first and second point from the end
+                const int e = l0 + (fl ? st : n * st), s1 = fl ? st : -st;
+                const bool end = l == 1 || l == n;
+                const double c0 = end ? -11. : -3.0, c1 = end ? 18. : -10.0, c2 = end ? -9. : 18.0, c3 = end ? 2. : -6.0;
+                const double den = end ? 6.0 : 12.0, rden = end ? 1.0 / 6.0 : 1.0 / 12.0;
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    const double *u = F.f[m == 3 ? F_T : F_U + m] + e;
+                    double du = c0 * __ldg(u) + c1 * __ldg(u + s1) + c2 * __ldg(u + 2 * s1) + c3 * __ldg(u + 3 * s1);
+                    const double u4 = __ldg(u + 4 * s1);
+                    if (!end) du = du + u4;
+                    F.f[F_DUV0 + m + 4 * d][id] = div_by(fl ? du : -du, den, rden);
+                }
             }
         }
     }
@@ -74,238 +104,293 @@ void launch_node_derivatives(const LaunchCtx &c) {
 // ---------------------------------------------------------------------------
 // viscous line flux
 // ---------------------------------------------------------------------------
-struct VisLine {
-    long long l0;  // field index of position 0 on the line
-    long long st;
-    int n;
-    bool fl, fr;
-};
-
-// Shared-memory staging of one line: VIS_NF values per point l = -1 .. n+2
-// (slot l+1): u, v, w, T; the 8 node derivatives along the two other
-// directions; the 9 metrics in the order kcx,etx,ctx,kcy,ety,cty,kcz,etz,ctz;
-// vol; the two Sutherland viscosities.  Then the line's viscous flux, 5 x (n+1).
-constexpr int VIS_NF = 24;
-constexpr int VIS_MAX_LINES = 32;  // lines per CTA (short k-lines are grouped many to a CTA)
-// 384 threads: the half-node fluxes of two 129-point lines (260) in one pass;
-// two CTAs per SM at 80 registers
-constexpr int VIS_THREADS = 320;
+// One CTA marches along NL lines, C half nodes at a time: thread (c, ln) forms the
+// viscous flux at half node h0 + c of line ln, then the flux difference at a point.
+// VIS_NF quantities of the points h0-1 .. h0+C+1 are in a ring in shared memory:
+// u, v, w, T, the 8 node derivatives along the two other directions, the 9 metrics
+// in the order kcx,etx,ctx,kcy,ety,cty,kcz,etz,ctz, vol and the two viscosities;
+// the next C points replace the oldest while the differences are formed.
+//
+// What bounds it: latency, of loads above all (staging and storing alone were 82 %
+// of the kernel that staged whole lines; FP64 pipe 13-16 % busy, DRAM 20 %).  So
+//   - a chunk of C = 8 half nodes leaves room for 16 lines in a CTA: 128 contiguous
+//     bytes per load across the lines, where 3 to 5 whole lines were 24 to 40 (the
+//     sectors read from L2 were four times the bytes used in the j direction);
+//   - the copies are asynchronous and need no registers, four CTAs of 128 registers
+//     fit an SM, and the old residual is read ahead of the barrier;
+//   - a point's quantities lie together, so a thread reaches all of them, 16 bytes at
+//     a time, from one address; the pitch is 2 mod 4: eight lanes' 16 bytes never
+//     share a bank;
+//   - formulas of the ends run in their own threads, not for a warp's every line.
+// Measured with the node derivatives, per step: channel (24 blocks, 4.2 M points)
+// 3110 us before, 1370 now; 64 small blocks (0.9 M points) 872 and 393 us; the plate
+// (8 blocks, 0.23 M points) 217 and 117 us.  Other splits over the channel: C = 10
+// 1437 us, C = 16 with 256 threads 1541, 64 threads 1804, 96 registers with spills
+// 1948; a ring that prefetches one chunk more (and holds fewer warps) 1861.
+constexpr int VIS_NF = 24, VIS_PITCH = 26, VIS_FP = 4;
+constexpr int VIS_THREADS = 128, VIS_CTAS = 4, VIS_CMAX = 8;
+constexpr int VIS_MAX_LINES = 32;  // lines per CTA
 enum : int { VS_U = 0, VS_DN = 4, VS_MET = 12, VS_VOL = 21, VS_V1 = 22, VS_V2 = 23 };
 
-__host__ __device__ inline int vis_line_stride(int n) {
-    // doubles per line, padded to 2 mod 16 so that the lines of a group fall
-    // on different banks when consecutive threads walk consecutive lines
-    int raw = VIS_NF * (n + 4) + 5 * (n + 1);
-    return (raw + 13) / 16 * 16 + 2;
+// A line of n points has n+1 half nodes in nch chunks of C; the first one takes the
+// remainder, so that the half nodes near the right end have a full chunk of points.
+__host__ __device__ inline int vis_chunk(int n) {
+    const int H = n + 1, nch = (H + VIS_CMAX - 1) / VIS_CMAX;
+    return (H + nch - 1) / nch;
+}
+__host__ __device__ inline int vis_ring(int n) {  // points in the ring
+    const int w = vis_chunk(n) + 3;
+    return w < n + 4 ? w : n + 4;
+}
+// lanes of a row of the ring: odd for i-lines, whose loads walk along a line
+__host__ __device__ inline int vis_row(int dir, int nl) { return dir == 0 ? nl | 1 : nl; }
+
+__device__ __forceinline__ void copy8_async(double *dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
 // out == nullptr: dq -= re*dFv in place; otherwise re*dFv is stored in
-// out[m*stride + point] for an ordered combine (k_combine_dq).  Two CTAs of
-// 320 threads per SM, 96 registers with almost no spill: 3.30 ms per channel
-// step for the three directions, against 3.40 at 384 threads and 80
-// registers, 4.07 at three CTAs of 256 and 5.30 at one CTA of 512.
+// out[m*stride + point] for an ordered combine (k_combine_dq).
 template <int dir>
-__global__ void __launch_bounds__(VIS_THREADS, 2) k_rhs_vis(DevParams P, DevFields F, const DevBlock *__restrict__ blocks,
-                                                    const LineGroup *__restrict__ groups, int hmax, double *out,
-                                                    long long stride) {
-    extern __shared__ double smem[];
+__global__ void __launch_bounds__(VIS_THREADS, VIS_CTAS) k_rhs_vis(DevParams P, DevFields F, const DevBlock *__restrict__ blocks,
+                                                    const LineGroup *__restrict__ groups, double *out, long long stride) {
+    extern __shared__ __align__(16) double smem[];
     const LineGroup G = groups[blockIdx.x];
     const DevBlock B = blocks[G.blk];
-    const int n = dimof(B, dir);
-    const int H = n + 1, W = n + 4;
-    const int NL = G.nl;
-    const int LS = vis_line_stride(n);
-    __shared__ VisLine lines[VIS_MAX_LINES];
-    const int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
-    if (threadIdx.x < NL) {
-        int c[3];
-        c[a1] = G.a0 + threadIdx.x;
-        c[a2] = G.b;
-        c[dir] = 0;
-        VisLine L;
-        L.l0 = gidx(B, c[0], c[1], c[2]);
-        L.st = dstride(B, dir);
-        L.n = n;
-        double rl = F.f[F_R][L.l0 - 2 * L.st], rr = F.f[F_R][L.l0 + (long long)(n + 3) * L.st];
-        L.fl = rl < 0.0 ? true : (F.f[F_T][L.l0 - 2 * L.st] < 0.0);
-        L.fr = rr < 0.0 ? true : (F.f[F_T][L.l0 + (long long)(n + 3) * L.st] < 0.0);
-        lines[threadIdx.x] = L;
+    const int n = dimof(B, dir), NL = G.nl, NLP = vis_row(dir, NL);
+    const int H = n + 1, C = vis_chunk(n), RP = vis_ring(n), FR = C + 5;
+    double *fv = smem + RP * NLP * VIS_PITCH;  // the last FR half nodes' fluxes
+    __shared__ int flags[VIS_MAX_LINES];       // bit 0: the left end has a boundary, bit 1: the right end
+    constexpr int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
+    const int st = (int)dstride(B, dir);
+    int o[3];
+    o[a1] = G.a0;
+    o[a2] = G.b;
+    o[dir] = 0;
+    const int base = (int)gidx(B, o[0], o[1], o[2]);          // position 0 of the first line
+    const int lstep = (int)dstride(B, a1);                    // to the next line
+    if ((int)threadIdx.x < 2 * NL) {
+        const int ln = threadIdx.x >> 1, right = threadIdx.x & 1;
+        const int g = base + ln * lstep + (right ? n + 3 : -2) * st;
+        const bool f = F.f[F_R][g] < 0.0 || F.f[F_T][g] < 0.0;
+        const int other = __shfl_xor_sync(__activemask(), (int)f, 1);
+        if (!right) flags[ln] = (f ? 1 : 0) | (other ? 2 : 0);
     }
-    __syncthreads();
-    const bool posmajor = (dir == 0);
-    const FastDiv dNL = fast_div_init(NL), dW = fast_div_init(W);
-    // ---- stage the line inputs: one thread per (line, point), all VIS_NF
-    // loads of the point issued back to back (coalesced along the line for
-    // i-lines, across the group's neighbouring lines otherwise)
-    {
-        const int g0 = dir == 0 ? 1 : 0, g1 = dir == 2 ? 1 : 2;  // the two other directions
-        for (int e = threadIdx.x; e < NL * W; e += blockDim.x) {
-            const int qq = posmajor ? fdiv(e, dW) : fdiv(e, dNL);
-            const int ln = posmajor ? qq : e - qq * NL;
-            const int p = posmajor ? e - qq * W : qq;
-            const VisLine &L = lines[ln];
-            const int l = p - 1;
-            const long long gi = L.l0 + (long long)l * L.st;
-            const bool inner = l >= 1 && l <= n;
-            double v[VIS_NF];
+    // this thread's half node and line; its point and line in the loads and stores,
+    // which walk along the line for i-lines and across the lines otherwise
+    const int c = threadIdx.x / NL, ln = threadIdx.x - c * NL;
+    const int pc = dir == 0 ? threadIdx.x % C : c, pl = dir == 0 ? threadIdx.x / C : ln;
+    const bool work = c < C, mover = dir == 0 ? pl < NL : c < C;
+    const int pbase = base + pl * lstep;
+    auto wrap = [](int x, int m) { return x >= m ? x - m : x; };
+    auto load = [&](int lo, int hi, int slo) {  // points lo..hi into the ring, from slot slo on
+        if (mover)
+            for (int p = lo + pc; p <= hi; p += C) {
+                constexpr int g0 = dir == 0 ? 1 : 0, g1 = dir == 2 ? 1 : 2;  // the two other directions
+                const int gi = pbase + p * st;
+                double *S = smem + (wrap(slo + p - lo, RP) * NLP + pl) * VIS_PITCH;
 #pragma unroll
-            for (int m = 0; m < 4; m++) v[VS_U + m] = __ldg(F.f[m == 3 ? F_T : F_U + m] + gi);
+                for (int m = 0; m < 4; m++) copy8_async(S + VS_U + m, F.f[m == 3 ? F_T : F_U + m] + gi);
+                if (p >= 1 && p <= n) {
 #pragma unroll
-            for (int m = 0; m < 4; m++) {
-                v[VS_DN + m] = inner ? __ldg(F.f[F_DUV0 + m + 4 * g0] + gi) : 0.0;
-                v[VS_DN + 4 + m] = inner ? __ldg(F.f[F_DUV0 + m + 4 * g1] + gi) : 0.0;
-            }
+                    for (int m = 0; m < 4; m++) {
+                        copy8_async(S + VS_DN + m, F.f[F_DUV0 + m + 4 * g0] + gi);
+                        copy8_async(S + VS_DN + 4 + m, F.f[F_DUV0 + m + 4 * g1] + gi);
+                    }
 #pragma unroll
-            for (int c = 0; c < 9; c++)  // kcx,etx,ctx,kcy,... = F_KCX + 3*(c%3) + c/3
-                v[VS_MET + c] = inner ? __ldg(F.f[F_KCX + 3 * (c % 3) + c / 3] + gi) : 0.0;
-            v[VS_VOL] = inner ? __ldg(F.f[F_VOL] + gi) : 0.0;
-            // viscosity at the point, as the reference's visl/vist arrays:
-            // mu + vist and mu*cp_prl + vist*cp_prt (vist = 0 when laminar)
-            const double mu = inner ? sutherland(P, v[VS_U + 3]) : 0.0;
-            const double vt = (inner && F.f[F_VIST]) ? __ldg(F.f[F_VIST] + gi) : 0.0;
-            v[VS_V1] = inner ? mu + vt : 0.0;
-            v[VS_V2] = inner ? mu * B.cp_prl + vt * B.cp_prt : 0.0;
-            double *S = smem + (size_t)ln * LS + p;
-#pragma unroll
-            for (int f = 0; f < VIS_NF; f++) S[f * W] = v[f];
-        }
-    }
-    __syncthreads();
-    // ---- per half node: viscous flux fv (line-fastest in every direction, so
-    // that the lanes of a warp share a position and its control path)
-    for (int idx = threadIdx.x; idx < NL * H; idx += blockDim.x) {
-        const int h = fdiv(idx, dNL);
-        const int ln = idx - h * NL;
-        const VisLine &L = lines[ln];
-        const double *S = smem + (size_t)ln * LS;
-        auto at = [&](int f, int x) { return S[f * W + x + 1]; };
-        // (u,v,w,T) at the half node: VALUE_line_half_virtual
-        double uh[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            auto Q = [&](int x) { return at(VS_U + m, x); };
-            double v;
-            if (n <= NIJK2ND) v = 0.5 * (Q(h) + Q(h + 1));
-            else if (L.fl && h == 0) v = (35.0 * Q(1) + -35.0 * Q(2) + 21.0 * Q(3) + -5.0 * Q(4)) / 16.0;
-            else if (L.fl && h == 1) v = (5.0 * Q(1) + 15.0 * Q(2) + -5.0 * Q(3) + 1.0 * Q(4)) / 16.0;
-            else if (L.fr && h == n) v = (35.0 * Q(n) + -35.0 * Q(n - 1) + 21.0 * Q(n - 2) + -5.0 * Q(n - 3)) / 16.0;
-            else if (L.fr && h == n - 1) v = (5.0 * Q(n) + 15.0 * Q(n - 1) + -5.0 * Q(n - 2) + 1.0 * Q(n - 3)) / 16.0;
-            else v = (9.0 * (Q(h) + Q(h + 1)) + -1.0 * (Q(h + 2) + Q(h - 1))) / 16.0;
-            uh[m] = v;
-        }
-        // derivatives at the half node: own direction from DUVWT_half_line_virtual,
-        // the two others interpolated from node derivatives
-        double dh[12];
-#pragma unroll
-        for (int g = 0; g < 3; g++) {
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                double v;
-                if (g == dir) {
-                    auto Q = [&](int x) { return at(VS_U + m, x); };
-                    if (n <= NIJK2ND) v = Q(h + 1) - Q(h);
-                    else if (L.fl && h == 0) v = (-71.0 * Q(1) + 141.0 * Q(2) + -93.0 * Q(3) + 23.0 * Q(4)) / 24.0;
-                    else if (L.fl && h == 1) v = (-22.0 * Q(1) + 17.0 * Q(2) + 9.0 * Q(3) + -5.0 * Q(4) + 1.0 * Q(5)) / 24.0;
-                    else if (L.fr && h == n) v = -(-71.0 * Q(n) + 141.0 * Q(n - 1) + -93.0 * Q(n - 2) + 23.0 * Q(n - 3)) / 24.0;
-                    else if (L.fr && h == n - 1) v = -(-22.0 * Q(n) + 17.0 * Q(n - 1) + 9.0 * Q(n - 2) + -5.0 * Q(n - 3) + 1.0 * Q(n - 4)) / 24.0;
-                    else v = (27.0 * (Q(h + 1) - Q(h)) + -1.0 * (Q(h + 2) - Q(h - 1))) / 24.0;
-                } else {
-                    const int slot = VS_DN + 4 * (g < dir ? g : g - 1) + m;
-                    auto D = [&](int x) { return at(slot, x); };
-                    v = value_half_node_ijk_at(D, n, h);
+                    for (int q = 0; q < 9; q++)  // kcx,etx,ctx,kcy,... = F_KCX + 3*(q%3) + q/3
+                        copy8_async(S + VS_MET + q, F.f[F_KCX + 3 * (q % 3) + q / 3] + gi);
+                    copy8_async(S + VS_VOL, F.f[F_VOL] + gi);
+                    copy8_async(S + VS_V1, F.f[F_MU] + gi);
+                    copy8_async(S + VS_V2, F.f[F_MU + 1] + gi);
                 }
-                dh[m + 4 * g] = v;
             }
-        }
-        // metrics (kcx,etx,ctx,kcy,ety,cty,kcz,etz,ctz), volume, viscosities
-        double kh[9];
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int h0 = 0, len = H - (H - 1) / C * C;       // this chunk's half nodes h0 .. h0+len-1
+    int have = len + 1 < 5 ? 5 : len + 1;        // the last point loaded: the left end's formulas reach point 5
+    if (have > n + 2) have = n + 2;
+    int hs = 0, fs = 0;                          // slots of point h0-1 and of half node h0
+    int done = 0;                                // the last point whose difference is out
+    load(-1, have, 0);
+    for (;;) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        const int lhi = h0 + len == H ? n : h0 + len - 3;  // differences this chunk completes: done+1 .. lhi
+        // the old residual of this thread's point, ahead of the barrier
+        double old[4];
+        const int l1 = done + 1 + pc, gi1 = pbase + l1 * st;
+        const bool out1 = mover && l1 <= lhi;
+        if (out1 && !out) {
 #pragma unroll
-        for (int c = 0; c < 9; c++) {
-            auto Q = [&](int x) { return at(VS_MET + c, x); };
-            kh[c] = value_half_node_at(Q, n, h);
+            for (int m = 0; m < 4; m++) old[m] = F.f[F_DQ2 + m][gi1];
         }
-        double volh, v1h, v2h;
-        {
-            auto Q = [&](int x) { return at(VS_VOL, x); };
-            auto V1 = [&](int x) { return at(VS_V1, x); };
-            auto V2 = [&](int x) { return at(VS_V2, x); };
-            volh = value_half_node_at(Q, n, h);
-            v1h = value_half_node_at(V1, n, h);
-            v2h = value_half_node_at(V2, n, h);
-        }
-        // DUVWT_DXYZ
-        double dx[12];
+        if (work && c < len) {
+            const int h = h0 + c;
+            // at the half node: (u,v,w,T) by VALUE_line_half_virtual, the derivatives
+            // along the own direction by DUVWT_half_line_virtual and along the two
+            // others interpolated from node derivatives, the metrics
+            // (kcx,etx,ctx,kcy,ety,cty,kcz,etz,ctz), volume and viscosities
+            double uh[4], dh[12], kh[9], volh, v1h, v2h;
+            auto set = [&](int f, double v) {  // staged quantity f (a constant): its value at the half node
+                if (f < VS_DN) uh[f] = v;
+                else if (f < VS_MET) {
+                    const int g = (f - VS_DN) / 4, gd = g < dir ? g : g + 1;
+                    dh[(f - VS_DN) % 4 + 4 * gd] = v;
+                } else if (f < VS_VOL) kh[f - VS_MET] = v;
+                else if (f == VS_VOL) volh = v;
+                else if (f == VS_V1) v1h = v;
+                else v2h = v;
+            };
+            auto at = [&](int p) { return smem + (wrap(hs + p + 1 - h0, RP) * NLP + ln) * VIS_PITCH; };
+            auto at2 = [&](int p) { return (const double2 *)at(p); };
+            if (n <= NIJK2ND) {
+                double t[VIS_NF];
+#pragma unroll 1
+                for (int f = 0; f < VIS_NF; f++) {
+                    auto Q = [&](int p) { return at(p)[f]; };
+                    t[f] = f >= VS_MET ? value_half_node_at(Q, n, h) : f >= VS_DN ? value_half_node_ijk_at(Q, n, h) : 0.5 * (Q(h) + Q(h + 1));
+                }
 #pragma unroll
-        for (int m = 1; m <= 3; m++) {
-            int m1 = m + m + m - 2, m2 = m1 + 1, m3 = m2 + 1;
-            dx[m - 1] = (kh[m1 - 1] * dh[0] + kh[m2 - 1] * dh[4] + kh[m3 - 1] * dh[8]) / volh;
-            dx[m + 2] = (kh[m1 - 1] * dh[1] + kh[m2 - 1] * dh[5] + kh[m3 - 1] * dh[9]) / volh;
-            dx[m + 5] = (kh[m1 - 1] * dh[2] + kh[m2 - 1] * dh[6] + kh[m3 - 1] * dh[10]) / volh;
-            dx[m + 8] = (kh[m1 - 1] * dh[3] + kh[m2 - 1] * dh[7] + kh[m3 - 1] * dh[11]) / volh;
-        }
-        // FLUX_VIS_LINE_new
-        double vs = v1h;
-        double vscc = vs * P.cc23;
-        double dudx = dx[0], dudy = dx[1], dudz = dx[2];
-        double dvdx = dx[3], dvdy = dx[4], dvdz = dx[5];
-        double dwdx = dx[6], dwdy = dx[7], dwdz = dx[8];
-        double t1 = vscc * (2.0 * dudx - dvdy - dwdz);
-        double t5 = vscc * (2.0 * dvdy - dwdz - dudx);
-        double t9 = vscc * (2.0 * dwdz - dudx - dvdy);
-        double t2 = vs * (dudy + dvdx);
-        double t3 = vs * (dudz + dwdx);
-        double t6 = vs * (dvdz + dwdy);
-        double kcp = v2h;
-        const double nx = dir == 0 ? kh[0] : dir == 1 ? kh[1] : kh[2];
-        const double ny = dir == 0 ? kh[3] : dir == 1 ? kh[4] : kh[5];
-        const double nz = dir == 0 ? kh[6] : dir == 1 ? kh[7] : kh[8];
-        double f1 = t1 * nx + t2 * ny + t3 * nz;
-        double f2 = t2 * nx + t5 * ny + t6 * nz;
-        double f3 = t3 * nx + t6 * ny + t9 * nz;
-        double f4 = uh[0] * f1 + uh[1] * f2 + uh[2] * f3 + kcp * (dx[9] * nx + dx[10] * ny + dx[11] * nz);
-        double *fv = smem + (size_t)ln * LS + (size_t)VIS_NF * W;
-        fv[0 * H + h] = 0.0;
-        fv[1 * H + h] = f1;
-        fv[2 * H + h] = f2;
-        fv[3 * H + h] = f3;
-        fv[4 * H + h] = f4;
-    }
-    __syncthreads();
-    // ---- per point: FLUX_DXYZ and dq -= re*dfv
-    for (int idx = threadIdx.x; idx < NL * n; idx += blockDim.x) {
-        const int l0 = fdiv(idx, dNL);
-        const int ln = idx - l0 * NL;
-        const int l = 1 + l0;
-        const VisLine &L = lines[ln];
-        const double *fv = smem + (size_t)ln * LS + (size_t)VIS_NF * W;
-        long long gi = L.l0 + (long long)l * L.st;
+                for (int f = 0; f < VIS_NF; f++) set(f, t[f]);
 #pragma unroll
-        for (int m = 0; m < 5; m++) {
-            auto fa = [&](int hh) { return fv[m * H + hh]; };
-            double dfv = flux_dxyz_at(fa, n, l);
-            if (out) {
-                out[m * stride + gi] = P.re * dfv;
+                for (int m = 0; m < 4; m++) dh[m + 4 * dir] = at(h + 1)[m] - at(h)[m];
             } else {
-                double *dq = F.f[F_DQ1 + m];
-                dq[gi] = dq[gi] - P.re * dfv;
+                const bool left = h <= 1, near = left || h >= n - 1, end = h == 0 || h == n;
+                const bool flag = near && (flags[ln] & (left ? 1 : 2));
+                if (!flag) {  // u, v, w, T with the points around the half node
+                    const double2 *qa = at2(h - 1), *qb = at2(h), *qc = at2(h + 1), *qd = at2(h + 2);
+#pragma unroll
+                    for (int q = 0; q < VS_DN / 2; q++) {
+                        const double2 va = qa[q], vb = qb[q], vc = qc[q], vd = qd[q];
+                        set(2 * q, (9.0 * (vb.x + vc.x) + -1.0 * (vd.x + va.x)) / 16.0);
+                        set(2 * q + 1, (9.0 * (vb.y + vc.y) + -1.0 * (vd.y + va.y)) / 16.0);
+                        dh[2 * q + 4 * dir] = div_by(27.0 * (vc.x - vb.x) + -1.0 * (vd.x - va.x), 24.0, 1.0 / 24.0);
+                        dh[2 * q + 1 + 4 * dir] = div_by(27.0 * (vc.y - vb.y) + -1.0 * (vd.y - va.y), 24.0, 1.0 / 24.0);
+                    }
+                }
+                if (!near) {
+                    const double2 *qa = at2(h - 1), *qb = at2(h), *qc = at2(h + 1), *qd = at2(h + 2);
+#pragma unroll
+                    for (int q = VS_DN / 2; q < VIS_NF / 2; q++) {
+                        const double2 va = qa[q], vb = qb[q], vc = qc[q], vd = qd[q];
+                        set(2 * q, (9.0 * (vb.x + vc.x) + -1.0 * (vd.x + va.x)) / 16.0);
+                        set(2 * q + 1, (9.0 * (vb.y + vc.y) + -1.0 * (vd.y + va.y)) / 16.0);
+                    }
+                } else {  // the other quantities have no ghost values: one-sided from the end's four points
+                    const int e = left ? 1 : n, s1 = left ? 1 : -1;
+                    const double *qa = at(e), *qb = at(e + s1), *qc = at(e + 2 * s1), *qd = at(e + 3 * s1);
+                    const double ca = end ? 35.0 : 5.0, cb = end ? -35.0 : 15.0, cc = end ? 21.0 : -5.0, cd = end ? -5.0 : 1.0;
+#pragma unroll
+                    for (int f = VS_DN; f < VIS_NF; f++) set(f, (ca * qa[f] + cb * qb[f] + cc * qc[f] + cd * qd[f]) / 16.0);
+                    if (flag) {
+                        const double *qe = at(e + 4 * s1);
+                        const double da = end ? -71.0 : -22.0, db = end ? 141.0 : 17.0, dc = end ? -93.0 : 9.0, dd = end ? 23.0 : -5.0;
+#pragma unroll
+                        for (int f = 0; f < VS_DN; f++) {
+                            set(f, (ca * qa[f] + cb * qb[f] + cc * qc[f] + cd * qd[f]) / 16.0);
+                            double d = da * qa[f] + db * qb[f] + dc * qc[f] + dd * qd[f];
+                            if (!end) d = d + qe[f];
+                            dh[f + 4 * dir] = div_by(left ? d : -d, 24.0, 1.0 / 24.0);
+                        }
+                    }
+                }
             }
+            // DUVWT_DXYZ
+            const double rvol = 1.0 / volh;
+            double dx[12];
+#pragma unroll
+            for (int m = 1; m <= 3; m++) {
+                int m1 = m + m + m - 2, m2 = m1 + 1, m3 = m2 + 1;
+                dx[m - 1] = div_by(kh[m1 - 1] * dh[0] + kh[m2 - 1] * dh[4] + kh[m3 - 1] * dh[8], volh, rvol);
+                dx[m + 2] = div_by(kh[m1 - 1] * dh[1] + kh[m2 - 1] * dh[5] + kh[m3 - 1] * dh[9], volh, rvol);
+                dx[m + 5] = div_by(kh[m1 - 1] * dh[2] + kh[m2 - 1] * dh[6] + kh[m3 - 1] * dh[10], volh, rvol);
+                dx[m + 8] = div_by(kh[m1 - 1] * dh[3] + kh[m2 - 1] * dh[7] + kh[m3 - 1] * dh[11], volh, rvol);
+            }
+            // FLUX_VIS_LINE_new
+            double vs = v1h;
+            double vscc = vs * P.cc23;
+            double dudx = dx[0], dudy = dx[1], dudz = dx[2];
+            double dvdx = dx[3], dvdy = dx[4], dvdz = dx[5];
+            double dwdx = dx[6], dwdy = dx[7], dwdz = dx[8];
+            double t1 = vscc * (2.0 * dudx - dvdy - dwdz);
+            double t5 = vscc * (2.0 * dvdy - dwdz - dudx);
+            double t9 = vscc * (2.0 * dwdz - dudx - dvdy);
+            double t2 = vs * (dudy + dvdx);
+            double t3 = vs * (dudz + dwdx);
+            double t6 = vs * (dvdz + dwdy);
+            double kcp = v2h;
+            const double nx = dir == 0 ? kh[0] : dir == 1 ? kh[1] : kh[2];
+            const double ny = dir == 0 ? kh[3] : dir == 1 ? kh[4] : kh[5];
+            const double nz = dir == 0 ? kh[6] : dir == 1 ? kh[7] : kh[8];
+            double f1 = t1 * nx + t2 * ny + t3 * nz;
+            double f2 = t2 * nx + t5 * ny + t6 * nz;
+            double f3 = t3 * nx + t6 * ny + t9 * nz;
+            double f4 = uh[0] * f1 + uh[1] * f2 + uh[2] * f3 + kcp * (dx[9] * nx + dx[10] * ny + dx[11] * nz);
+            double2 *w = (double2 *)(fv + (wrap(fs + c, FR) * NLP + ln) * VIS_FP);
+            w[0] = make_double2(f1, f2);  // the mass flux is zero
+            w[1] = make_double2(f3, f4);
         }
+        __syncthreads();
+        if (have < n + 2) {
+            int hi = h0 + len + C + 1;
+            if (hi > n + 2) hi = n + 2;
+            load(have + 1, hi, wrap(hs + have + 2 - h0, RP));
+            have = hi;
+        }
+        // FLUX_DXYZ and dq -= re*dfv
+        auto fslot = [&](int h) { return wrap(fs + h - h0 < 0 ? fs + h - h0 + FR : fs + h - h0, FR); };
+        if (mover)
+            for (int l = l1; l <= lhi; l += C) {
+                const int gi = pbase + l * st;
+                if (n > NIJK2ND && l > 2 && l < n - 1) {
+                    double f[6][4];
+#pragma unroll
+                    for (int q = 0; q < 6; q++) {
+                        const double2 *a = (const double2 *)(fv + (fslot(l - 3 + q) * NLP + pl) * VIS_FP);
+                        const double2 x = a[0], y = a[1];
+                        f[q][0] = x.x; f[q][1] = x.y; f[q][2] = y.x; f[q][3] = y.y;
+                    }
+#pragma unroll
+                    for (int m = 0; m < 4; m++) {
+                        const double dfv = div_by(2250.0 * (f[3][m] - f[2][m]) - 125.0 * (f[4][m] - f[1][m]) + 9.0 * (f[5][m] - f[0][m]),
+                                                  1920.0, 1.0 / 1920.0);
+                        if (out) out[(m + 1) * stride + gi] = P.re * dfv;
+                        else F.f[F_DQ2 + m][gi] = (l == l1 ? old[m] : F.f[F_DQ2 + m][gi]) - P.re * dfv;
+                    }
+                } else {
+#pragma unroll 1
+                    for (int m = 0; m < 4; m++) {
+                        const double *f = fv + pl * VIS_FP + m;
+                        auto fa = [&](int hh) { return f[fslot(hh) * NLP * VIS_FP]; };
+                        const double dfv = flux_dxyz_at(fa, n, l);
+                        if (out) out[(m + 1) * stride + gi] = P.re * dfv;
+                        else F.f[F_DQ2 + m][gi] = F.f[F_DQ2 + m][gi] - P.re * dfv;
+                    }
+                }
+            }
+        if (lhi == n) break;
+        if (lhi > done) done = lhi;
+        h0 += len;
+        hs = wrap(hs + len, RP);
+        fs = wrap(fs + len, FR);
+        len = C;
     }
-    (void)hmax;
 }
 
-size_t rhs_vis_line_bytes(int n) { return (size_t)vis_line_stride(n) * 8; }
-int rhs_vis_max_lines() { return VIS_MAX_LINES; }
-int rhs_vis_threads() { return VIS_THREADS; }
+size_t rhs_vis_line_bytes(int dir, int n, int nl) {
+    return sizeof(double) * (size_t)vis_row(dir, nl) * (vis_ring(n) * VIS_PITCH + VIS_FP * (vis_chunk(n) + 5));
+}
+int rhs_vis_lines(int n) { return std::min(VIS_MAX_LINES, VIS_THREADS / vis_chunk(n)); }
 
 void launch_rhs_vis(const LaunchCtx &c, int dir, cudaStream_t st, double *out) {
     if (c.mixed) return launch_rhs_vis_mx(c, dir, st, out);
     const DirTable &T = c.vis[dir];
     if (T.ngroups == 0) return;
     const long long stride = c.total;
-    if (dir == 0) k_rhs_vis<0><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.hmax, out, stride);
-    else if (dir == 1) k_rhs_vis<1><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.hmax, out, stride);
-    else k_rhs_vis<2><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.hmax, out, stride);
+    if (dir == 0) k_rhs_vis<0><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, out, stride);
+    else if (dir == 1) k_rhs_vis<1><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, out, stride);
+    else k_rhs_vis<2><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, out, stride);
 }
 
 void setup_rhs_vis_attrs(size_t max_smem) {

@@ -15,7 +15,7 @@ struct LineGroup {
 
 struct DirTable {
     LineGroup *groups = nullptr;  // device
-    int ngroups = 0, hmax = 0;
+    int ngroups = 0;
     size_t smem = 0;              // dynamic shared memory of the launch (max over groups)
 };
 
@@ -244,9 +244,8 @@ void launch_rhs_vis(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
 // all three directions of the viscous (vis = true) or inviscid residual
 void launch_rhs_dirs(const LaunchCtx &c, bool vis);
 void setup_rhs_vis_attrs(size_t max_smem);
-size_t rhs_vis_line_bytes(int n);  // shared memory of one line in k_rhs_vis
-int rhs_vis_max_lines();           // lines per CTA in k_rhs_vis
-int rhs_vis_threads();            // threads per CTA in k_rhs_vis
+size_t rhs_vis_line_bytes(int dir, int n, int nl);  // shared memory of nl lines in k_rhs_vis
+int rhs_vis_lines(int n);                           // lines per CTA in k_rhs_vis
 size_t adj_line_bytes(int n);     // shared memory of one line in the adjoint's kernels
 int adj_max_lines();              // lines per CTA in the adjoint's kernels
 // mixed-precision residual (k_rhs_mixed.cu)
