@@ -123,6 +123,7 @@ struct WcnsContext {
         if (pm_pool) cudaFree(pm_pool);
         if (sa_pool) cudaFree(sa_pool);
         if (adj_pool) cudaFree(adj_pool);
+        if (L.adj_rec) cudaFree(L.adj_rec);
         if (stage) cudaFree(stage);
         if (stage_first) cudaFree(stage_first);
         if (stream) cudaStreamDestroy(stream);
@@ -1785,6 +1786,13 @@ static int adj_ready(WcnsContext *c, const char *who) {
         const size_t bytes = sizeof(double) * 5 * (size_t)WCNS_ADJ_NSLOTS * (size_t)c->total;
         CK(cudaMalloc(&c->adj_pool, bytes));
         CK(cudaMemset(c->adj_pool, 0, bytes));
+        // the records of the LU-SGS operator, unless they would take more than a
+        // quarter of what is free: it goes plane by plane without them
+        size_t free_b = 0, all_b = 0;
+        const size_t rec = sizeof(double) * ADJ_REC_WORDS * (size_t)c->total_pm;
+        CK(cudaMemGetInfo(&free_b, &all_b));
+        if (adj_lu_marches(c->L) && rec <= free_b / 4 && cudaMalloc(&c->L.adj_rec, rec) == cudaSuccess) c->L.adj_rec_stride = c->total_pm;
+        cudaGetLastError();
     }
     return 0;
 }

@@ -30,8 +30,12 @@
 // of mxdq_std), so each transposed sweep is again a wavefront over planes.
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "wcns_dev.cuh"
 #include "wcns_launch.h"
+
+namespace cg = cooperative_groups;
 
 namespace wcns {
 
@@ -657,6 +661,176 @@ __global__ void __launch_bounds__(256) k_adj_lu(DevParams P, DevFields F, const 
     }
 }
 
+// The same sweeps as one launch each: a cluster of CTAs per block, a thread per
+// column (j,k), whose cell moves along i as the plane advances, and a cluster barrier
+// between planes.  What a cell needs of the state -- the split Jacobians of its three
+// directions for both signs, coed and its b -- is put into records first, all cells at
+// once (k_adj_lu_records), plane by plane and column by column, so that a warp reads
+// neighbouring words; in the fields the cells of a plane are a row apart and every
+// lane of a load touches its own sector.  What a cell hands to its j and k neighbours
+// (lower and upper sweep of P: the terms A x; of P^T: y = coed x) goes through the
+// same memory, along i it stays in registers.  A cell's next record is read between
+// the barrier's two halves.  x takes b's place in the record.
+// Bound by latency: 2 us per plane for the neighbours' terms from L2, three 5x5
+// products, the stores' way to L2 and the barrier.  A launch per plane spent 10 us on
+// each (launch, scattered loads, root and divisions, one after the other).  Operator
+// and transpose on a block of 65x33x17 points (113 planes): 2290 and 2440 us before,
+// 570 and 440 now; forming the Jacobians in the sweep from the fields, 1390 and 1300.
+enum : int { AR_U = 0, AR_V, AR_W, AR_H, AR_AF, AR_C2, AR_CE, AR_DIR };  // then per direction nx, ny, nz, ct and l1, x1, x2 of A+, of A-
+constexpr int AR_X = AR_DIR + 30, AR_EX = AR_X + 5;                      // b, then x; the neighbours' terms
+static_assert(AR_EX + 10 == ADJ_REC_WORDS, "words of a record");
+constexpr int ADJ_CLUSTER = BC_CLUSTER, ADJ_LU_THREADS = 512;
+
+__device__ __forceinline__ long long adj_slot_of(const DevBlock &B, int p, int col) {
+    return B.pmoff + (long long)(p - 3) * (B.nj * B.nk) + col;
+}
+
+__global__ void __launch_bounds__(128) k_adj_lu_records(DevParams P, DevFields F, const DevBlock *__restrict__ blocks, double *__restrict__ rec,
+                                                     long long rs, const double *__restrict__ b, long long stride) {
+    const DevBlock B = blocks[blockIdx.y];
+    const int ncol = B.nj * B.nk;
+    const long long nslot = (long long)(B.ni + B.nj + B.nk - 2) * ncol;
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nslot; q += (long long)gridDim.x * blockDim.x) {
+        const int p = (int)(q / ncol) + 3, col = (int)(q % ncol), j = col % B.nj + 1, k = col / B.nj + 1, i = p - j - k;
+        if (i < 1 || i > B.ni) continue;
+        const long long id = gidx(B, i, j, k);
+        double *R = rec + B.pmoff + q;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const Split A = split_at(P, F, id, d, 1), M = split_at(P, F, id, d, -1);
+            if (d == 0) {
+                R[AR_U * rs] = A.V[1];
+                R[AR_V * rs] = A.V[2];
+                R[AR_W * rs] = A.V[3];
+                R[AR_H * rs] = A.V[4];
+                R[AR_AF * rs] = A.b[0];
+                R[AR_C2 * rs] = A.c2;
+                R[AR_CE * rs] = coed_inv(F, id);
+            }
+            double *D = R + (AR_DIR + 10 * d) * rs;
+            D[0] = A.N[1];
+            D[rs] = A.N[2];
+            D[2 * rs] = A.N[3];
+            D[3 * rs] = A.N[4];
+            D[4 * rs] = A.l1;
+            D[5 * rs] = A.x1;
+            D[6 * rs] = A.x2;
+            D[7 * rs] = M.l1;
+            D[8 * rs] = M.x1;
+            D[9 * rs] = M.x2;
+        }
+#pragma unroll
+        for (int m = 0; m < 5; m++) R[(AR_X + m) * rs] = b[m * stride + id];
+    }
+}
+
+// x from the records back to the fields
+__global__ void __launch_bounds__(128) k_adj_lu_store(const DevBlock *__restrict__ blocks, const double *__restrict__ rec, long long rs, double *x,
+                                                   long long stride) {
+    const DevBlock B = blocks[blockIdx.y];
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < B.npts; q += (long long)gridDim.x * blockDim.x) {
+        int i, j, k;
+        decode_point(B, q, i, j, k);
+        const long long id = gidx(B, i, j, k), sl = adj_slot_of(B, i + j + k, (k - 1) * B.nj + j - 1);
+#pragma unroll
+        for (int m = 0; m < 5; m++) x[m * stride + id] = rec[(AR_X + m) * rs + sl];
+    }
+}
+
+// MODE as in k_adj_lu
+template <int MODE>
+__global__ void __launch_bounds__(ADJ_LU_THREADS) k_adj_lu_march(DevParams P, const DevBlock *__restrict__ blocks, double *rec, long long rs) {
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr bool up = MODE == 0 || MODE == 2;  // planes in ascending order
+    constexpr int sign = MODE == 0 || MODE == 3 ? 4 : 7;  // A+ or A-
+    const DevBlock B = blocks[blockIdx.x / ADJ_CLUSTER];
+    const int ncol = B.nj * B.nk, col = (int)cluster.block_rank() * blockDim.x + threadIdx.x;
+    const bool has = col < ncol;
+    const int j = has ? col % B.nj + 1 : 1, k = has ? col / B.nj + 1 : 1;
+    // neighbours this cell receives from and hands to, along j and k
+    const bool from[2] = {up ? j >= 2 : j <= B.nj - 1, up ? k >= 2 : k <= B.nk - 1};
+    const bool to[2] = {up ? j <= B.nj - 1 : j >= 2, up ? k <= B.nk - 1 : k >= 2};
+    const int p0 = up ? 3 : B.ni + B.nj + B.nk, np = B.ni + B.nj + B.nk - 2;
+    const double ae = P.gama - 1.0;
+    double c[AR_DIR], dr[3][7], bx[5], carry[5];
+    auto fetch = [&](int p) {
+        const double *R = rec + adj_slot_of(B, p, col);
+#pragma unroll
+        for (int q = 0; q < AR_DIR; q++) c[q] = R[q * rs];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+#pragma unroll
+            for (int q = 0; q < 7; q++) dr[d][q] = R[(AR_DIR + 10 * d + (q < 4 ? q : sign + q - 4)) * rs];
+#pragma unroll
+        for (int m = 0; m < 5; m++) bx[m] = R[(AR_X + m) * rs];
+    };
+    auto apply = [&](int d, const double *y, double *f) {
+        Split S;
+        const double *q = dr[d];
+        const double a[5] = {q[3], -q[0], -q[1], -q[2], 0.0}, b[5] = {c[AR_AF], -ae * c[AR_U], -ae * c[AR_V], -ae * c[AR_W], ae};
+        const double N[5] = {0.0, q[0], q[1], q[2], q[3]}, V[5] = {1.0, c[AR_U], c[AR_V], c[AR_W], c[AR_H]};
+        S.l1 = q[4];
+        S.x1 = q[5];
+        S.x2 = q[6];
+        S.c2 = c[AR_C2];
+#pragma unroll
+        for (int m = 0; m < 5; m++) { S.a[m] = a[m]; S.b[m] = b[m]; S.N[m] = N[m]; S.V[m] = V[m]; }
+        split_apply(S, y, f, MODE >= 2);
+    };
+    auto plane = [&](int s) { return up ? p0 + s : p0 - s; };
+    auto inside = [&](int p) { return has && p - j - k >= 1 && p - j - k <= B.ni; };
+    if (inside(p0)) fetch(p0);
+    for (int s = 0; s < np; s++) {
+        const int p = plane(s);
+        if (inside(p)) {
+            const int i = p - j - k;
+            double *R = rec + adj_slot_of(B, p, col);
+            const long long nb[2] = {(up ? 1LL : -1LL) * (ncol + 1), (up ? 1LL : -1LL) * (ncol + B.nj)};  // to the next plane's j and k neighbours
+            double e[2][5], acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, f[5], y[5];
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                if (from[q])  // the neighbour's y, or what it left here
+#pragma unroll
+                    for (int m = 0; m < 5; m++) e[q][m] = __ldcg(MODE >= 2 ? R + (AR_EX + m) * rs - nb[q] : R + (AR_EX + 5 * q + m) * rs);
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                if (d == 0 ? (up ? i < 2 : i > B.ni - 1) : !from[d - 1]) continue;
+#pragma unroll
+                for (int m = 0; m < 5; m++) y[m] = d == 0 ? carry[m] : e[d - 1][m];
+                if (MODE >= 2) apply(d, y, f);
+#pragma unroll
+                for (int m = 0; m < 5; m++) acc[m] += MODE >= 2 ? f[m] : y[m];
+            }
+            const double ce = c[AR_CE];
+#pragma unroll
+            for (int m = 0; m < 5; m++) {
+                const double v = MODE == 0 ? (-bx[m] + acc[m]) * ce : MODE == 1 ? bx[m] - acc[m] * ce : MODE == 2 ? bx[m] - acc[m] : bx[m] + acc[m];
+                y[m] = MODE >= 2 ? ce * v : v;
+                R[(AR_X + m) * rs] = MODE == 3 ? -y[m] : v;  // the last factor of P^T is -coed
+            }
+            if (MODE >= 2) {
+#pragma unroll
+                for (int m = 0; m < 5; m++) {
+                    carry[m] = y[m];
+                    __stcg(R + (AR_EX + m) * rs, y[m]);
+                }
+            } else {
+                apply(0, y, carry);
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                    if (to[q]) {
+                        apply(q + 1, y, f);
+#pragma unroll
+                        for (int m = 0; m < 5; m++) __stcg(R + (AR_EX + 5 * q + m) * rs + nb[q], f[m]);
+                    }
+            }
+        }
+        cluster.barrier_arrive();
+        if (s + 1 < np && inside(plane(s + 1))) fetch(plane(s + 1));
+        cluster.barrier_wait();
+    }
+}
+
 // pointwise over the interior: x = -coed x (the last factor of P^T), or
 // x = (d prim / d Q)^T x + g (conserved adjoint of a prim-space adjoint)
 template <int MODE>
@@ -790,6 +964,13 @@ void launch_rhs_invis_vjp(const LaunchCtx &c, const double *lam, double *out, bo
                                                                                                           out, c.total);
 }
 
+// a thread of the cluster for every column of the largest block
+bool adj_lu_marches(const LaunchCtx &c) {
+    int maxcols = 0;
+    for (int q = 0; q < c.nblocks; q++) maxcols = std::max(maxcols, c.hblocks[q].nj * c.hblocks[q].nk);
+    return maxcols <= ADJ_CLUSTER * ADJ_LU_THREADS;
+}
+
 void launch_lusgs_operator(const LaunchCtx &c, double *x, const double *b, bool transpose) {
     int maxcols = 0, pmax = 0;
     long long maxp = 0;
@@ -798,6 +979,24 @@ void launch_lusgs_operator(const LaunchCtx &c, double *x, const double *b, bool 
         maxcols = std::max(maxcols, B.nj * B.nk);
         pmax = std::max(pmax, B.ni + B.nj + B.nk);
         maxp = std::max(maxp, B.npts);
+    }
+    // one launch per sweep while a cluster has a thread for every column; larger
+    // blocks go plane by plane
+    if (c.adj_rec) {
+        const int threads = ((maxcols + ADJ_CLUSTER - 1) / ADJ_CLUSTER + 31) / 32 * 32;
+        const dim3 rg((unsigned)std::min<long long>(((long long)(maxcols) * (pmax - 2) + 127) / 128, 8192), c.nblocks);
+        k_adj_lu_records<<<rg, 128, 0, c.stream>>>(*c.P, *c.F, c.blocks, c.adj_rec, c.adj_rec_stride, b, c.total);
+        auto sweep = [&](auto kern) { launch_block_clusters(kern, c.nblocks, threads, c.stream, *c.P, c.blocks, c.adj_rec, c.adj_rec_stride); };
+        if (!transpose) {
+            sweep(k_adj_lu_march<0>);
+            sweep(k_adj_lu_march<1>);
+        } else {
+            sweep(k_adj_lu_march<2>);
+            sweep(k_adj_lu_march<3>);
+        }
+        const dim3 pg((unsigned)std::min<long long>((maxp + 127) / 128, 8192), c.nblocks);
+        k_adj_lu_store<<<pg, 128, 0, c.stream>>>(c.blocks, c.adj_rec, c.adj_rec_stride, x, c.total);
+        return;
     }
     const dim3 grid((unsigned)((maxcols + 255) / 256), c.nblocks);
     if (!transpose) {

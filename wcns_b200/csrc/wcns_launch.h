@@ -140,6 +140,10 @@ struct LaunchCtx {
     int *err = nullptr;            // device error slots
     DirTable inv[3], vis[3];
     DirTable adj[3];  // lines of the adjoint's inviscid operators
+    // records of the LU-SGS operator's sweeps (ADJ_REC_WORDS arrays of adj_rec_stride);
+    // null: the operator goes plane by plane
+    double *adj_rec = nullptr;
+    long long adj_rec_stride = 0;
     // mixed precision (wcns_set_precision(ctx, 32)): the residual kernels of
     // k_rhs_mixed.cu with their own line groups, and FP32 node derivatives
     // of (u,v,w,T) in the storage of the FP64 ones (12 x total floats)
@@ -248,6 +252,8 @@ size_t rhs_vis_line_bytes(int dir, int n, int nl);  // shared memory of nl lines
 int rhs_vis_lines(int n);                           // lines per CTA in k_rhs_vis
 size_t adj_line_bytes(int n);     // shared memory of one line in the adjoint's kernels
 int adj_max_lines();              // lines per CTA in the adjoint's kernels
+constexpr int ADJ_REC_WORDS = 52; // doubles per cell of the LU-SGS operator's records
+bool adj_lu_marches(const LaunchCtx &c);  // whether its sweeps can run on records
 // mixed-precision residual (k_rhs_mixed.cu)
 void launch_rhs_invis_mx(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
 void launch_rhs_vis_mx(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
