@@ -1207,7 +1207,7 @@ extern "C" int wcns_sa_setup(WcnsContext *c, const double *const *xyz, double ti
         CK(cudaMemset(c->sa_pool, 0, sizeof(double) * SA_NFIELDS * (size_t)c->total));
         double *f[SA_NFIELDS];
         for (int q = 0; q < SA_NFIELDS; q++) f[q] = c->sa_pool + (size_t)q * c->total;
-        c->SA = SaFields{f[0], f[1], f[2], f[3], f[4], {f[5], f[6], f[7]}};
+        c->SA = SaFields{f[0], f[1], f[2], f[3], f[4], {f[5], f[6], f[7]}, f[8]};
     }
     // constants as cal_rhs_source_SA evaluates its parameter statements
     const double cb1 = 0.1355, cb2 = 0.622, cv1 = 7.1, cga = 2. / 3.0, ki = 0.419, cw3 = 2.0;

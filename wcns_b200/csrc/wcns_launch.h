@@ -57,9 +57,9 @@ struct DevWall {
 // Spalart-Allmaras model arrays (one field each, the pool's layout): qke,
 // vist, the wall distance, and the model's dqke, spec and qke derivatives
 struct SaFields {
-    double *qke, *vist, *dist, *dqke, *spec, *dmu[3];
+    double *qke, *vist, *dist, *dqke, *spec, *dmu[3], *vis;
 };
-constexpr int SA_NFIELDS = 8;
+constexpr int SA_NFIELDS = 9;
 
 // SA constants as the reference evaluates them (cal_rhs_source_SA,
 // turblence.f90:2508-2513), computed on the host, and the $step/$turbulence
