@@ -355,6 +355,40 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
         for (int pass = 0; pass < 5; pass++) {  // 0 inviscid, 1 viscous, 2 and 3 the same in mixed precision, 4 the adjoint's operators
             std::vector<LineGroup> g;
             size_t sm_dir = 0;
+            int cmax = 0;
+            if (pass <= 1) {
+                // The FP64 kernels march along lines in chunks of at most cmax half
+                // nodes, 128 / cmax lines to a CTA.  8 is the fastest where there are
+                // CTAs enough for the chip: loads across the lines are 128 contiguous
+                // bytes (inviscid, channel of 4.2 M points: 1135 us, and 1206, 1481,
+                // 1813, 2127 for 16, 32, 64, 128).  On fewer points a CTA's chain of
+                // chunks is what takes time, and longer chunks of fewer lines give
+                // more CTAs with shorter chains (vortex of 65x33x17 points: 85 us with
+                // 8, then 67, 52, 46, 42).  Cost of a choice: the CTAs' chunks, two
+                // more each for its start, over the places on the chip, at the
+                // price of its loads, but no less than the longest chain.
+                double best = 1e300;
+                const double price[5] = {1.0, 1.06, 1.3, 1.6, 1.87};
+                for (int q = 0; q < 5; q++) {
+                    const int cm = 8 << q;
+                    double sum = 0.0, chain = 0.0;
+                    for (int b = 0; b < nbk; b++) {
+                        const DevBlock &D = c->blk[b].d;
+                        const int n = dimof(D, dir);
+                        if (pass == 0 && n <= NIJK2D) continue;
+                        const int na = dimof(D, dir == 0 ? 1 : 0), nb2 = dimof(D, dir == 2 ? 1 : 2);
+                        const int nl = std::max(1, pass == 0 ? std::min(inv_cap, rhs_invis_lines(n, cm)) : std::min(vis_cap, rhs_vis_lines(n, cm)));
+                        const double t = 2.0 + (pass == 0 ? rhs_invis_chunks(n, cm) : rhs_vis_chunks(n, cm));
+                        sum += t * nb2 * ((na + nl - 1) / nl);
+                        chain = std::max(chain, t);
+                    }
+                    const double cost = std::max(price[q] * sum / (4 * 148), chain);
+                    if (cost < best * 0.999) {
+                        best = cost;
+                        cmax = cm;
+                    }
+                }
+            }
             for (int b = 0; b < nbk; b++) {
                 const DevBlock &D = c->blk[b].d;
                 int n = dimof(D, dir);
@@ -363,56 +397,30 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
                 if (pass == 4 && (c->P.nvis != 0 || c->P.nscheme != 4)) continue;  // refused there
                 int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
                 int na = dimof(D, a1), nb2 = dimof(D, a2);
-                size_t per_line = pass == 0 ? rhs_invis_line_bytes(n, sections) : pass == 1 ? rhs_vis_line_bytes(dir, n, 1)
+                size_t per_line = pass == 0 || pass == 1 ? 0
                                 : pass == 2 ? rhs_invis_mx_line_bytes(n) : pass == 3 ? rhs_vis_mx_line_bytes(n) : adj_line_bytes(n);
-                // staged lines per CTA: the kernel's share of the SM's shared memory for
-                // the FP64 inviscid kernel, 72 KB for the mixed-precision kernels and the
-                // adjoint's; the FP64 viscous kernel takes as many as its threads
-                int NL = pass == 0 ? std::max(1, std::min({std::min(inv_cap, rhs_invis_max_lines()), 3072 / (5 * (n + 2)),
-                                                           (int)(rhs_invis_smem() / per_line)}))
-                       : pass == 1 ? std::max(1, std::min(vis_cap, rhs_vis_lines(n)))
+                // the FP64 kernels take as many lines as their threads, the others stage
+                // at most 72 KB
+                int NL = pass == 0 ? std::max(1, std::min(inv_cap, rhs_invis_lines(n, cmax)))
+                       : pass == 1 ? std::max(1, std::min(vis_cap, rhs_vis_lines(n, cmax)))
                        : pass == 2 || pass == 4 ? std::max(1, std::min({std::min(inv_cap, pass == 2 ? rhs_invis_mx_max_lines() : adj_max_lines()),
                                                                         3072 / (5 * (n + 2)), (int)((72 * 1024) / per_line)}))
                                    : std::max(1, std::min({std::min(vis_cap, rhs_vis_mx_max_lines()), 512 / (n + 1), (int)((72 * 1024) / per_line)}));
-                if (pass == 1) {  // rows of equal share
+                if (pass <= 1) {  // rows of equal share
                     const int ng = (na + NL - 1) / NL;
                     NL = (na + ng - 1) / ng;
-                }
-                if (pass == 0) {
-                    // the heavy phase has one item per (line, half node), and 13 more
-                    // per end with boundary sections: of NL/2..NL lines take the count
-                    // whose items fill the last pass of the CTA's threads best, so that
-                    // few threads idle at the barrier after it
-                    const int thr = rhs_invis_threads();
-                    int per = n + 1;
-                    if (sections)
-                        for (int lr = -1; lr <= 1; lr += 2)
-                            for (const HReg &R : c->blk[b].regs)
-                                if ((R.bctype == 4 || R.bctype == 2) && R.s_nd == dir + 1 && R.s_lr == lr) {
-                                    per += 13;
-                                    break;
-                                }
-                    int best = NL;
-                    double best_fill = 0.0;
-                    for (int q = NL; q >= std::max(1, (NL + 1) / 2); q--) {
-                        const int items = q * per, rounds = (items + thr - 1) / thr;
-                        const double fill = (double)items / ((double)rounds * thr);
-                        if (fill > best_fill + 1e-9) {
-                            best_fill = fill;
-                            best = q;
-                        }
-                    }
-                    NL = best;
                 }
                 for (int bb = 1; bb <= nb2; bb++)
                     for (int a = 1; a <= na; a += NL) {
                         LineGroup lg{b, a, bb, std::min(NL, na - a + 1)};
                         g.push_back(lg);
-                        sm_dir = std::max(sm_dir, pass == 1 ? rhs_vis_line_bytes(dir, n, lg.nl) : per_line * lg.nl);
+                        sm_dir = std::max(sm_dir, pass == 0 ? rhs_invis_line_bytes(dir, n, lg.nl, cmax, sections)
+                                                : pass == 1 ? rhs_vis_line_bytes(dir, n, lg.nl, cmax) : per_line * lg.nl);
                     }
             }
             DirTable &T = pass == 0 ? L.inv[dir] : pass == 1 ? L.vis[dir] : pass == 2 ? L.inv_mx[dir] : pass == 3 ? L.vis_mx[dir] : L.adj[dir];
             T.ngroups = (int)g.size();
+            T.cmax = cmax;
             T.smem = sm_dir;
             if (T.groups) {  // a rebuild (wcns_set_shape): the old table goes
                 c->owned.erase(std::remove(c->owned.begin(), c->owned.end(), (void *)T.groups), c->owned.end());

@@ -8,67 +8,80 @@
 // Van Leer (flux.f90:395-501) or Roe (flux.f90:116-244) fluxes, and
 // FLUX_DXYZ (WCNSE5.f90:209-254).  dq += dF.
 //
-// One CTA owns a group of NL lines of one block, staged in shared memory.  The
-// reference's sequential line loop is split into two parallel phases:
+// One CTA marches along a group of NL lines of one block, C half nodes at a time
+// (cmax in wcns_launch.h), over a ring of points in shared memory.  Per chunk:
 //   A  per half node: the left state (weights centred at point h) and the right
 //      state (point h+1), boundary closures, positivity fallback, numerical
-//      flux; plus the 26 independent fluxes of the nscheme=41/42 boundary
-//      sections, in lines that have one;
+//      flux; at a flagged end also the 13 independent fluxes of the
+//      nscheme=41/42 boundary sections;
 //   B  per point: sixth-order flux difference (or the boundary-section
-//      difference where the reference overrides it) accumulated into dq.
+//      difference where the reference overrides it) accumulated into dq, while
+//      the next points arrive (asynchronous copies).
 //
-// What bounds it: the FP64 operations of phase A and, before anything, their
-// divisions (124 cycles each, a dozen instructions).  So
+// What bounds it: the FP64 operations of phase A (the pipe is busy half of the
+// time), and the latency around them.  So
 //   - the nonlinear weights are formed over a common denominator: with
 //     E = (eps + IS)^2, w_k = C_k / E_k / sum(C / E) = C_k prod_{j != k} E_j / S,
-//     one division per state instead of six.  E is between eps^2 = 1e-12 and
-//     q^4, so the products stay far inside the exponent range;
+//     one division per state instead of six (124 cycles each, a dozen
+//     instructions).  E is between eps^2 = 1e-12 and q^4, so the products stay far
+//     inside the exponent range;
 //   - a half node's two states are formed by the thread that evaluates its
 //     flux: the smoothness indicators are computed twice, but nothing of them
-//     goes through shared memory and one barrier less separates the phases;
+//     goes through shared memory;
 //   - a reciprocal whose last bit does not matter takes five instructions
 //     (recip), a quotient that does, by a constant, three (div_by);
 //   - the code of the few half nodes near a flagged end is kept out of the way
 //     and in one copy for the five variables: unrolled it was as long as the
-//     rest, and a quarter of the warps' time went into instruction fetches.
-// Before, with a thread's states unrolled for every closure and six divisions
-// each, the FP64 pipe was busy 25-37 % and the warps waited 5.4 cycles per
-// instruction for code.  Measured per step, before and now: channel 3540 and
-// 1500 us, 64 small blocks 1543 and 535 us, one block of 121x75x51 points (Roe)
-// 347 and 190 us, the plate 265 and 148 us, one vortex 73 and 57 us.
+//     rest, and a quarter of the warps' time went into instruction fetches;
+//   - whole lines in shared memory leave room for three to seven of them, loads
+//     across the lines then fetch twice the bytes they use, and staging,
+//     arithmetic and stores follow one another; a ring of a chunk and its halo
+//     leaves room for 16 lines.
+// Measured per step, with the closures unrolled and whole lines; the code above on
+// whole lines; now: channel (24 blocks, 4.2 M points, Roe, nscheme 41) 3540, 1511,
+// 1135 us; 64 small blocks (0.9 M points) 1543, 539, 470; one block of 121x75x51
+// points (nscheme 4) 347, 190, 167; the plate (0.23 M points) 265, 148, 116; one
+// vortex of 65x33x17 73, 57, 42.  Three, five, six CTAs per SM over the channel:
+// 1228, 1216, 1323 us; two of 256 threads with C = 16 1300.
 // The central part of the fluxes and the differences keep the reference's
 // operations and their order: where the flow is uniform they cancel to
 // round-off, which is compared.  The weights, and in the Roe flux all that is
 // multiplied by the jump, are free of that.
+#include <algorithm>
+
 #include "wcns_dev.cuh"
 #include "wcns_launch.h"
 
 namespace wcns {
 
-struct InvLine {
-    const double *sq;  // shared-memory copy of the prim line: sq[m*(n+6) + l+2], l = -2..n+3
-    const double *sk;  // shared-memory copy of the metrics (kx,ky,kz) of the line: sk[c*n + l-1], l = 1..n
-    long long stride;
-    long long dqbase;  // field index of point l=0 on the line (point l at dqbase + l*stride)
-    int n, ist, ied;
-};
+// The ring: the five variables of the points h0-2 .. h0+C+2 and, at 1..n, the
+// metrics of this direction, one point's eight values after the other.
+constexpr int INV_PITCH = 10, INV_FP = 6;
+constexpr int INV_THREADS = 128, INV_CTAS = 4;
+constexpr int INV_MAX_LINES = 32;  // lines per CTA
 
-__device__ __forceinline__ double qv(const InvLine &L, int m, int l) { return L.sq[m * (L.n + 6) + l + 2]; }
-
-// 80 registers and 72 KB of staged lines per CTA, 24 warps per SM.  Against four
-// CTAs of 256 threads at 64 registers: 1500 instead of 1544 us per step over the
-// channel (24 blocks, 4.2 M points, Roe, nscheme 41), 535 instead of 513 us over
-// 64 small blocks (0.9 M points), 57 instead of 63 us over a vortex of 65x33x17.
-constexpr int INV_THREADS = 256, INV_CTAS = 3;
-constexpr int INV_MAX_LINES = 32;  // lines per CTA (short lines are grouped many to a CTA)
-
-// doubles of shared memory per line: prim 5 x (n+6), metrics 3 x n, f 5 x (n+1)
-// and, with boundary sections, their 26 fluxes; padded to 2 mod 16 so that the
-// lines of a group fall on different banks
-__host__ __device__ inline int inv_line_stride(int n, bool sections) {
-    int raw = 5 * (n + 6) + 3 * n + 5 * (n + 1) + (sections ? 130 : 0);
-    return (raw + 13) / 16 * 16 + 2;
+// A line of n points has n+1 half nodes in nch chunks of C; the first one takes the
+// remainder, so that all that the right end's formulas reach lies in the last chunk's
+// points.  Short lines are one chunk: both ends' sections reach the other end there.
+__host__ __device__ inline int inv_chunk(int n, int cmax) {
+    const int H = n + 1;
+    if (H <= 13) return H;
+    const int nch = (H + cmax - 1) / cmax;
+    return (H + nch - 1) / nch;
 }
+// lanes of a row of the ring: odd for i-lines, whose loads walk along a line
+__host__ __device__ inline int inv_row(int dir, int nl) { return dir == 0 ? nl | 1 : nl; }
+
+struct InvLine {  // one line's view of the ring
+    const double *ring;  // point p at slot wrap(s0 + p - p0), NLP * INV_PITCH apart
+    int p0, s0, RP, step;
+    int n, ist, ied;
+    __device__ __forceinline__ const double *at(int p) const {
+        int s = s0 + p - p0;
+        if (s >= RP) s -= RP;
+        return ring + s * step;
+    }
+};
 
 // The state at a half node from the five points around `c0` (WCNSE5.f90:2-206):
 // left states from point h, right states from point h+1.
@@ -106,10 +119,9 @@ __constant__ double sec_table[SEC_ROWS * SEC_W] = {
 #undef SEC_ROW
 
 // state of variable m from a row: points 1..4, or n..n-3 for the right end
-__device__ __forceinline__ double sec_state(const double *row, const double *q, int m, int n, bool right) {
-    const double *x = q + m * (n + 6) + (right ? n + 2 : 3);
-    const int d = right ? -1 : 1;
-    return div_by(row[0] * x[0] + row[1] * x[d] + row[2] * x[2 * d] + row[3] * x[3 * d], row[4], row[5]);
+__device__ __forceinline__ double sec_state(const double *row, const InvLine &L, int m, bool right) {
+    const int e = right ? L.n : 1, d = right ? -1 : 1;
+    return div_by(row[0] * L.at(e)[m] + row[1] * L.at(e + d)[m] + row[2] * L.at(e + 2 * d)[m] + row[3] * L.at(e + 3 * d)[m], row[4], row[5]);
 }
 
 // Where a half node's left state comes from near a flagged end: the row of its
@@ -127,91 +139,108 @@ __device__ __forceinline__ int closure_right(const InvLine &L, int h, bool &end)
     return L.ied < L.n && h >= L.n - 2 ? SEC_C + L.n - h : -1;
 }
 
+__device__ __forceinline__ void inv_copy8(double *dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
 // dq += dF in place.
 template <int dir, int NFLUX>
 __global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(DevParams P, DevFields F, const DevBlock *__restrict__ blocks,
-                                                       const LineGroup *__restrict__ groups, int *err) {
-    extern __shared__ double smem[];
+                                                       const LineGroup *__restrict__ groups, int cmax, int *err) {
+    extern __shared__ __align__(16) double smem[];
     const LineGroup G = groups[blockIdx.x];
     const DevBlock B = blocks[G.blk];
-    const int n = dimof(B, dir);
-    const int H = n + 1, W = n + 6;
-    const int NL = G.nl;
+    const int n = dimof(B, dir), NL = G.nl, NLP = inv_row(dir, NL);
+    const int H = n + 1, C = inv_chunk(n, cmax), RP = C + 5, FR = C + 5;
     const bool scheme4x = P.nscheme == 41 || P.nscheme == 42;
-    const int LS = inv_line_stride(n, scheme4x);
-    const int wf = 5 * W + 3 * n, wsec = wf + 5 * H;  // flux, section fluxes within a line
-    __shared__ InvLine lines[INV_MAX_LINES];
-    __shared__ int flagged;  // a line of the group has a boundary section
+    double *fr = smem + RP * NLP * INV_PITCH;   // the last FR half nodes' fluxes
+    double *secf = fr + FR * NLP * INV_FP;      // 26 section fluxes per line
+    __shared__ int flags[INV_MAX_LINES];        // bit 0: the left end has a boundary, bit 1: the right end
     __shared__ double sec[SEC_ROWS * SEC_W];
-    if (threadIdx.x == 0) flagged = 0;
     if (threadIdx.x < SEC_ROWS * SEC_W) sec[threadIdx.x] = sec_table[threadIdx.x];
-    __syncthreads();
-    const int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
-    if (threadIdx.x < NL) {
-        int c[3];
-        c[a1] = G.a0 + threadIdx.x;
-        c[a2] = G.b;
-        c[dir] = -2;
-        long long base = gidx(B, c[0], c[1], c[2]);
-        InvLine L;
-        L.sq = smem + (size_t)threadIdx.x * LS;
-        L.sk = L.sq + (size_t)5 * W;
-        L.stride = dstride(B, dir);
-        L.dqbase = base + 2 * L.stride;
-        L.n = n;
-        L.ist = __ldg(F.f[F_R] + base) < SMALL ? 2 : 0;
-        L.ied = __ldg(F.f[F_R] + base + (long long)(n + 5) * L.stride) < SMALL ? n - 2 : n;
-        lines[threadIdx.x] = L;
-        if (scheme4x && (L.ist > 1 || L.ied < n)) flagged = 1;
+    static_assert(SEC_ROWS * SEC_W <= INV_THREADS, "the table is copied in one go");
+    constexpr int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
+    const int st = (int)dstride(B, dir), lstep = (int)dstride(B, a1);
+    int o3[3];
+    o3[a1] = G.a0;
+    o3[a2] = G.b;
+    o3[dir] = 0;
+    const int base = (int)gidx(B, o3[0], o3[1], o3[2]);  // position 0 of the first line
+    // this thread's half node and line; its point and line in the loads and stores,
+    // which walk along the line for i-lines and across the lines otherwise
+    const int TC = INV_THREADS / NL, c = threadIdx.x / NL, ln = threadIdx.x - c * NL;
+    const int pc = dir == 0 ? threadIdx.x % C : c, pl = dir == 0 ? threadIdx.x / C : ln;
+    const bool mover = dir == 0 ? pl < NL : c < C;
+    const int pbase = base + pl * lstep;
+    auto wrap = [](int x, int m) { return x >= m ? x - m : x; };
+    auto load = [&](int lo, int hi, int slo) {  // points lo..hi into the ring, from slot slo on
+        if (mover)
+            for (int p = lo + pc; p <= hi; p += C) {
+                const int gi = pbase + p * st;
+                double *S = smem + (wrap(slo + p - lo, RP) * NLP + pl) * INV_PITCH;
+#pragma unroll
+                for (int m = 0; m < 5; m++) inv_copy8(S + m, F.f[F_R + m] + gi);
+                if (p >= 1 && p <= n) {
+#pragma unroll
+                    for (int q = 0; q < 3; q++) inv_copy8(S + 5 + q, F.f[F_KCX + 3 * dir + q] + gi);
+                }
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int h0 = 0, len = H - (H - 1) / C * C;  // this chunk's half nodes h0 .. h0+len-1
+    int have = len + 2 < 7 ? 7 : len + 2;   // the last point loaded: the left end's sections reach point 7
+    if (have > n + 3) have = n + 3;
+    int hs = 0, fs = 0;                     // slots of point h0-2 and of half node h0
+    int done = 0;                           // the last point whose difference is out
+    load(-2, have, 0);
+    int anyl = 0, anyr = 0;                 // a line has a boundary section at its left, right end
+    if ((int)threadIdx.x < NL) {
+        const int g = base + threadIdx.x * lstep;
+        anyl = __ldg(F.f[F_R] + g - 2 * st) < SMALL;
+        anyr = __ldg(F.f[F_R] + g + (n + 3) * st) < SMALL;
+        flags[threadIdx.x] = anyl | anyr << 1;
     }
-    __syncthreads();
-    constexpr bool posmajor = (dir == 0);
-    const FastDiv dNL = fast_div_init(NL), dW = fast_div_init(W), dn = fast_div_init(n);
-    // ---- stage the prim line (l = -2..n+3) and the metrics of this
-    // direction (l = 1..n): one thread per (line, point), coalesced along the
-    // line for i-lines and across the group's neighbouring lines otherwise
-    for (int e = threadIdx.x; e < NL * W; e += blockDim.x) {
-        const int qq = posmajor ? fdiv(e, dW) : fdiv(e, dNL);
-        const int ln = posmajor ? qq : e - qq * NL;
-        const int p = posmajor ? e - qq * W : qq;
-        const long long gi = lines[ln].dqbase + (long long)(p - 2) * lines[ln].stride;
-        double v[8];
+    anyl = __syncthreads_or(scheme4x && anyl);
+    anyr = __syncthreads_or(scheme4x && anyr);
+    const double gama1 = P.gama - 1.0, gama1_1 = 1.0 / gama1;
+    int nbad = 0;
+    InvLine L;
+    L.ring = smem + ln * INV_PITCH;
+    L.RP = RP;
+    L.step = NLP * INV_PITCH;
+    L.n = n;
+    L.ist = flags[ln] & 1 ? 2 : 0;
+    L.ied = flags[ln] & 2 ? n - 2 : n;
+    for (;;) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        const bool last = h0 + len == H;
+        const int lhi = last ? n : h0 + len - 3;  // differences this chunk completes: done+1 .. lhi
+        // the old residual of this thread's point, ahead of the barrier
+        double old[5];
+        const int l1 = done + 1 + pc, gi1 = pbase + l1 * st;
+        if (mover && l1 <= lhi) {
 #pragma unroll
-        for (int m = 0; m < 5; m++) v[m] = __ldg(F.f[F_R + m] + gi);
-        const bool inner = p >= 3 && p <= n + 2;
-#pragma unroll
-        for (int c = 0; c < 3; c++) v[5 + c] = inner ? __ldg(F.f[F_KCX + 3 * dir + c] + gi) : 0.0;
-        double *sq = smem + (size_t)ln * LS;
-#pragma unroll
-        for (int m = 0; m < 5; m++) sq[m * W + p] = v[m];
-        if (inner) {
-#pragma unroll
-            for (int c = 0; c < 3; c++) sq[5 * W + c * n + p - 3] = v[5 + c];
+            for (int m = 0; m < 5; m++) old[m] = F.f[F_DQ1 + m][gi1];
         }
-    }
-    __syncthreads();
-    // Phase A walks the items line-fastest in every direction: the lanes of a
-    // warp take the same position on neighbouring lines and follow one control
-    // path, and items without work (boundary sections of a line that has none)
-    // gather into whole warps that skip them.
-    {
-        const int NT = H + (flagged ? 26 : 0);
-        const double gama1 = P.gama - 1.0, gama1_1 = 1.0 / gama1;
-        int nbad = 0;
-        for (int idx = threadIdx.x; idx < NL * NT; idx += blockDim.x) {
-            const int t = fdiv(idx, dNL);
-            const int ln = idx - t * NL;
-            const InvLine &L = lines[ln];
+        L.p0 = h0 - 2;
+        L.s0 = hs;
+        // the half nodes, then the sections of the ends in the chunk: items
+        // line-fastest, the lanes of a warp take the same position on neighbouring
+        // lines and follow one control path
+        const int nl13 = h0 == 0 && anyl ? 13 : 0, T = len + nl13 + (last && anyr ? 13 : 0);
+        for (int t = c; t < T && c < TC; t += TC) {
             double ql[5], qr[5], fl[5];
             // Where the two states come from: a row of the table (and the end it
             // counts from) or, -1, the interior scheme.  Sections 0..25: at the
             // left end s1 at half nodes 0..3, s2 at 1..5, s3 at 1..4; at the right
             // end s4, s5, s6 likewise, counting down from n.
-            int h = t, rowl = -1, rowr = -1;
+            int h = h0 + t, rowl = -1, rowr = -1, isec = -1;
             bool endl = false, endr = false;
-            if (t >= H) {
-                int sidx = t - H;
+            if (t >= len) {
+                int sidx = t - len + (nl13 ? 0 : 13);
                 const bool right = sidx >= 13;
+                isec = sidx;
                 if (right ? L.ied >= n : L.ist <= 1) continue;
                 if (right) sidx -= 13;
                 const int s1 = P.nscheme == 42 ? SEC_S1_42 : SEC_S1;
@@ -244,112 +273,130 @@ __global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(DevParams P
             }
             if (rowl < 0) rowl = closure_left(L, h, endl);
             if (rowr < 0) rowr = closure_right(L, h, endr);
+            const double *x0 = L.at(h - 2), *x1 = L.at(h - 1), *x2 = L.at(h), *x3 = L.at(h + 1), *x4 = L.at(h + 2), *x5 = L.at(h + 3);
             if (rowl < 0 && rowr < 0) {
 #pragma unroll
                 for (int m = 0; m < 5; m++) {
-                    const double *q = L.sq + m * W + h + 2;
-                    const double q0 = q[-2], q1 = q[-1], q2 = q[0], q3 = q[1], q4 = q[2], q5 = q[3];
-                    ql[m] = wcns_state<true>(q0, q1, q2, q3, q4);
-                    qr[m] = wcns_state<false>(q1, q2, q3, q4, q5);
+                    ql[m] = wcns_state<true>(x0[m], x1[m], x2[m], x3[m], x4[m]);
+                    qr[m] = wcns_state<false>(x1[m], x2[m], x3[m], x4[m], x5[m]);
                 }
             } else {  // few items: one copy of the code for all variables
                 double tl[5], tr[5];
 #pragma unroll 1
                 for (int m = 0; m < 5; m++) {
-                    const double *q = L.sq + m * W + h + 2;
-                    tl[m] = rowl < 0 ? wcns_state<true>(q[-2], q[-1], q[0], q[1], q[2]) : sec_state(sec + rowl * SEC_W, L.sq, m, n, endl);
-                    tr[m] = rowr < 0 ? wcns_state<false>(q[-1], q[0], q[1], q[2], q[3]) : sec_state(sec + rowr * SEC_W, L.sq, m, n, endr);
+                    tl[m] = rowl < 0 ? wcns_state<true>(x0[m], x1[m], x2[m], x3[m], x4[m]) : sec_state(sec + rowl * SEC_W, L, m, endl);
+                    tr[m] = rowr < 0 ? wcns_state<false>(x1[m], x2[m], x3[m], x4[m], x5[m]) : sec_state(sec + rowr * SEC_W, L, m, endr);
                 }
 #pragma unroll
                 for (int m = 0; m < 5; m++) { ql[m] = tl[m]; qr[m] = tr[m]; }
             }
             // positivity fallback: the neighbouring point; in s1 and s4 means
             const bool badl = ql[0] <= RMIN_LIMIT || ql[4] <= PMIN_LIMIT, badr = qr[0] <= RMIN_LIMIT || qr[4] <= PMIN_LIMIT;
-            const bool same = t >= H && rowl == rowr && rowl < SEC_S2;
+            const bool same = isec >= 0 && rowl == rowr && rowl < SEC_S2;
             if (badl || badr) {
                 const int ia = h > 1 ? h : 1, ib = h + 1 < n ? h + 1 : n;
                 // points of the means; of the neighbours
                 const int la = same && endl ? 1 : ia, lb = same ? (endl ? h : h + 1) : ia, ra = same ? la : ib, rb = same ? lb : ib;
 #pragma unroll
-                for (int m = 0; m < 5; m++) {
-                    if (badl) ql[m] = (qv(L, m, la) + qv(L, m, lb)) / 2.0;
-                    if (badr) qr[m] = (qv(L, m, ra) + qv(L, m, rb)) / 2.0;
+                for (int m = 0; m < 5; m++) {  // from memory: a mean may reach the line's first point
+                    const double *q = F.f[F_R + m] + base + ln * lstep;
+                    if (badl) ql[m] = (q[la * st] + q[lb * st]) / 2.0;
+                    if (badr) qr[m] = (q[ra * st] + q[rb * st]) / 2.0;
                 }
             }
             // half-node metrics: VALUE_HALF_NODE of (kx,ky,kz) along the line
-            auto ax = [&](int l) { return L.sk[l - 1]; };
-            auto ay = [&](int l) { return L.sk[n + l - 1]; };
-            auto az = [&](int l) { return L.sk[2 * n + l - 1]; };
-            double kx = value_half_node_at(ax, n, h), ky = value_half_node_at(ay, n, h), kz = value_half_node_at(az, n, h);
+            double kx, ky, kz;
+            if (h > 1 && h < n - 1) {
+                kx = (9.0 * (x2[5] + x3[5]) + -1.0 * (x4[5] + x1[5])) / 16.0;
+                ky = (9.0 * (x2[6] + x3[6]) + -1.0 * (x4[6] + x1[6])) / 16.0;
+                kz = (9.0 * (x2[7] + x3[7]) + -1.0 * (x4[7] + x1[7])) / 16.0;
+            } else {  // from the end's four points
+                const bool right = h >= n - 1, end = h == 0 || h == n;
+                const int e = right ? n : 1, d = right ? -1 : 1;
+                const double *ka = L.at(e), *kb = L.at(e + d), *kc = L.at(e + 2 * d), *kd = L.at(e + 3 * d);
+                const double ca = end ? 35.0 : 5.0, cb = end ? -35.0 : 15.0, cc = end ? 21.0 : -5.0, cd = end ? -5.0 : 1.0;
+                kx = (ca * ka[5] + cb * kb[5] + cc * kc[5] + cd * kd[5]) / 16.0;
+                ky = (ca * ka[6] + cb * kb[6] + cc * kc[6] + cd * kd[6]) / 16.0;
+                kz = (ca * ka[7] + cb * kb[7] + cc * kc[7] + cd * kd[7]) / 16.0;
+            }
             const double kt = 0.0;  // kct=0, so every half-node value of kt is +0
             if (NFLUX == 3) nbad += flux_roe(P, gama1_1, ql, qr, kx, ky, kz, kt, same, fl);
             else nbad += flux_split<NFLUX>(P, ql, qr, kx, ky, kz, kt, fl);
-            double *f_ = smem + (size_t)ln * LS;
-            if (t < H) {
-                f_ += wf + h;
+            double *f_ = isec < 0 ? fr + (wrap(fs + h - h0, FR) * NLP + ln) * INV_FP : secf + (ln * 26 + isec) * 5;
 #pragma unroll
-                for (int m = 0; m < 5; m++) f_[m * H] = fl[m];
-            } else {
-                f_ += wsec + (t - H) * 5;
-#pragma unroll
-                for (int m = 0; m < 5; m++) f_[m] = fl[m];
-            }
+            for (int m = 0; m < 5; m++) f_[m] = fl[m];
         }
-        if (nbad) atomicAdd(&err[ERR_ROE], nbad);
-    }
-    __syncthreads();
-    // ---- phase B: flux difference and accumulation into dq, per (line, point),
-    // in the order of memory: along the line for i-lines, across the
-    // neighbouring lines otherwise
-    for (int idx = threadIdx.x; idx < NL * n; idx += blockDim.x) {
-        const int qq = posmajor ? fdiv(idx, dn) : fdiv(idx, dNL);
-        const int ln = posmajor ? qq : idx - qq * NL;
-        const int l = 1 + (posmajor ? idx - qq * n : qq);
-        const InvLine &L = lines[ln];
-        const long long gi = L.dqbase + (long long)l * L.stride;
-        const double *f_ = smem + (size_t)ln * LS + wf;
-        const double *sc = smem + (size_t)ln * LS + wsec;
-        const bool right = scheme4x && L.ied < n && l >= n - 2, left = scheme4x && L.ist > 1 && l <= 3;
-        if (!right && !left && l > 2 && l < n - 1) {
-            double old[5];
-#pragma unroll
-            for (int m = 0; m < 5; m++) old[m] = F.f[F_DQ1 + m][gi];
-#pragma unroll
-            for (int m = 0; m < 5; m++) {
-                const double *f = f_ + m * H + l;
-                F.f[F_DQ1 + m][gi] = old[m] + div_by(2250.0 * (f[0] - f[-1]) - 125.0 * (f[1] - f[-2]) + 9.0 * (f[2] - f[-3]), 1920.0, 1.0 / 1920.0);
-            }
-            continue;
+        __syncthreads();
+        if (have < n + 3) {  // the next chunk's points, in place of the oldest
+            int hi = h0 + len + C + 2;
+            if (hi > n + 3) hi = n + 3;
+            load(have + 1, hi, wrap(hs + have + 3 - h0, RP));
+            have = hi;
         }
+        // flux difference and accumulation into dq, in the order of memory: along
+        // the line for i-lines, across the neighbouring lines otherwise
+        auto fslot = [&](int h) { return wrap(fs + h - h0 < 0 ? fs + h - h0 + FR : fs + h - h0, FR); };
+        if (mover) {
+            const int fl = flags[pl];
+            for (int l = l1; l <= lhi; l += C) {
+                const int gi = pbase + l * st;
+                const bool right = scheme4x && (fl & 2) && l >= n - 2, left = scheme4x && (fl & 1) && l <= 3;
+                if (l != l1) {
+#pragma unroll
+                    for (int m = 0; m < 5; m++) old[m] = F.f[F_DQ1 + m][gi];
+                }
+                if (!right && !left && l > 2 && l < n - 1) {
+                    const double *q[6];
+#pragma unroll
+                    for (int x = 0; x < 6; x++) q[x] = fr + (fslot(l - 3 + x) * NLP + pl) * INV_FP;
+#pragma unroll
+                    for (int m = 0; m < 5; m++)
+                        F.f[F_DQ1 + m][gi] = old[m] + div_by(2250.0 * (q[3][m] - q[2][m]) - 125.0 * (q[4][m] - q[1][m]) + 9.0 * (q[5][m] - q[0][m]),
+                                                             1920.0, 1.0 / 1920.0);
+                    continue;
+                }
+                const double *sc = secf + pl * 130;
+                double df[5];
 #pragma unroll 1
-        for (int m = 0; m < 5; m++) {
-            double df;
-            if (right) {
-                const double *s4 = sc + 13 * 5 + m, *s5 = sc + 17 * 5 + m, *s6 = sc + 22 * 5 + m;
-                // section fluxes f(ni-h): s4[k] holds f(k), s5[k] and s6[k] hold f(k+1)
-                if (l == n) df = -(-23.0 * s4[0] + 21.0 * s4[5] + 3.0 * s4[10] - 1.0 * s4[15]) / 24.0;
-                else if (l == n - 1) df = -(-22.0 * s5[0] + 17.0 * s5[5] + 9.0 * s5[10] - 5.0 * s5[15] + s5[20]) / 24.0;
-                else df = -(s6[0] - 27.0 * s6[5] + 27.0 * s6[10] - s6[15]) / 24.0;
-            } else if (left) {
-                const double *s1 = sc + m, *s2 = sc + 4 * 5 + m, *s3 = sc + 9 * 5 + m;
-                if (l == 1) df = (-23.0 * s1[0] + 21.0 * s1[5] + 3.0 * s1[10] - 1.0 * s1[15]) / 24.0;
-                else if (l == 2) df = (-22.0 * s2[0] + 17.0 * s2[5] + 9.0 * s2[10] - 5.0 * s2[15] + s2[20]) / 24.0;
-                else df = (s3[0] - 27.0 * s3[5] + 27.0 * s3[10] - s3[15]) / 24.0;
-            } else {
-                auto fa = [&](int hh) { return f_[m * H + hh]; };
-                df = flux_dxyz_at(fa, n, l);
+                for (int m = 0; m < 5; m++) {
+                    double v;
+                    if (right) {
+                        const double *s4 = sc + 13 * 5 + m, *s5 = sc + 17 * 5 + m, *s6 = sc + 22 * 5 + m;
+                        // section fluxes f(ni-h): s4[k] holds f(k), s5[k] and s6[k] hold f(k+1)
+                        if (l == n) v = -(-23.0 * s4[0] + 21.0 * s4[5] + 3.0 * s4[10] - 1.0 * s4[15]) / 24.0;
+                        else if (l == n - 1) v = -(-22.0 * s5[0] + 17.0 * s5[5] + 9.0 * s5[10] - 5.0 * s5[15] + s5[20]) / 24.0;
+                        else v = -(s6[0] - 27.0 * s6[5] + 27.0 * s6[10] - s6[15]) / 24.0;
+                    } else if (left) {
+                        const double *s1 = sc + m, *s2 = sc + 4 * 5 + m, *s3 = sc + 9 * 5 + m;
+                        if (l == 1) v = (-23.0 * s1[0] + 21.0 * s1[5] + 3.0 * s1[10] - 1.0 * s1[15]) / 24.0;
+                        else if (l == 2) v = (-22.0 * s2[0] + 17.0 * s2[5] + 9.0 * s2[10] - 5.0 * s2[15] + s2[20]) / 24.0;
+                        else v = (s3[0] - 27.0 * s3[5] + 27.0 * s3[10] - s3[15]) / 24.0;
+                    } else {
+                        auto fa = [&](int hh) { return fr[(fslot(hh) * NLP + pl) * INV_FP + m]; };
+                        v = flux_dxyz_at(fa, n, l);
+                    }
+                    df[m] = v;
+                }
+#pragma unroll
+                for (int m = 0; m < 5; m++) F.f[F_DQ1 + m][gi] = old[m] + df[m];
             }
-            F.f[F_DQ1 + m][gi] = F.f[F_DQ1 + m][gi] + df;
         }
+        if (last) break;
+        if (lhi > done) done = lhi;
+        h0 += len;
+        hs = wrap(hs + len, RP);
+        fs = wrap(fs + len, FR);
+        len = C;
     }
+    if (nbad) atomicAdd(&err[ERR_ROE], nbad);
 }
 
 template <int NFLUX>
 static void launch_invis(const LaunchCtx &c, int dir, cudaStream_t st) {
     const DirTable &T = c.inv[dir];
-    if (dir == 0) k_rhs_invis<0, NFLUX><<<T.ngroups, INV_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, c.err);
-    else if (dir == 1) k_rhs_invis<1, NFLUX><<<T.ngroups, INV_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, c.err);
-    else k_rhs_invis<2, NFLUX><<<T.ngroups, INV_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, c.err);
+    if (dir == 0) k_rhs_invis<0, NFLUX><<<T.ngroups, INV_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.cmax, c.err);
+    else if (dir == 1) k_rhs_invis<1, NFLUX><<<T.ngroups, INV_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.cmax, c.err);
+    else k_rhs_invis<2, NFLUX><<<T.ngroups, INV_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.cmax, c.err);
 }
 
 void launch_rhs_invis(const LaunchCtx &c, int dir, cudaStream_t st, double *out) {
@@ -373,9 +420,11 @@ void setup_rhs_invis_attrs(size_t max_smem, int nflux) {
     else set_invis_attrs<3>((int)max_smem);
 }
 
-size_t rhs_invis_line_bytes(int n, bool sections) { return (size_t)inv_line_stride(n, sections) * 8; }
-int rhs_invis_threads() { return INV_THREADS; }
-size_t rhs_invis_smem() { return (size_t)(216 * 1024 / INV_CTAS); }
-int rhs_invis_max_lines() { return INV_MAX_LINES; }
+size_t rhs_invis_line_bytes(int dir, int n, int nl, int cmax, bool sections) {
+    const int C = inv_chunk(n, cmax);
+    return sizeof(double) * ((size_t)inv_row(dir, nl) * (C + 5) * (INV_PITCH + INV_FP) + (sections ? (size_t)nl * 130 : 0));
+}
+int rhs_invis_lines(int n, int cmax) { return std::min(INV_MAX_LINES, INV_THREADS / inv_chunk(n, cmax)); }
+int rhs_invis_chunks(int n, int cmax) { return (n + inv_chunk(n, cmax)) / inv_chunk(n, cmax); }
 
 }  // namespace wcns

@@ -113,7 +113,7 @@ void launch_node_derivatives(const LaunchCtx &c) {
 //
 // What bounds it: latency, of loads above all (staging and storing alone were 82 %
 // of the kernel that staged whole lines; FP64 pipe 13-16 % busy, DRAM 20 %).  So
-//   - a chunk of C = 8 half nodes leaves room for 16 lines in a CTA: 128 contiguous
+//   - a chunk of C = 8 half nodes (cmax) leaves room for 16 lines in a CTA: 128 contiguous
 //     bytes per load across the lines, where 3 to 5 whole lines were 24 to 40 (the
 //     sectors read from L2 were four times the bytes used in the j direction);
 //   - the copies are asynchronous and need no registers, four CTAs of 128 registers
@@ -128,18 +128,18 @@ void launch_node_derivatives(const LaunchCtx &c) {
 // 1437 us, C = 16 with 256 threads 1541, 64 threads 1804, 96 registers with spills
 // 1948; a ring that prefetches one chunk more (and holds fewer warps) 1861.
 constexpr int VIS_NF = 24, VIS_PITCH = 26, VIS_FP = 4;
-constexpr int VIS_THREADS = 128, VIS_CTAS = 4, VIS_CMAX = 8;
+constexpr int VIS_THREADS = 128, VIS_CTAS = 4;
 constexpr int VIS_MAX_LINES = 32;  // lines per CTA
 enum : int { VS_U = 0, VS_DN = 4, VS_MET = 12, VS_VOL = 21, VS_V1 = 22, VS_V2 = 23 };
 
 // A line of n points has n+1 half nodes in nch chunks of C; the first one takes the
 // remainder, so that the half nodes near the right end have a full chunk of points.
-__host__ __device__ inline int vis_chunk(int n) {
-    const int H = n + 1, nch = (H + VIS_CMAX - 1) / VIS_CMAX;
+__host__ __device__ inline int vis_chunk(int n, int cmax) {
+    const int H = n + 1, nch = (H + cmax - 1) / cmax;
     return (H + nch - 1) / nch;
 }
-__host__ __device__ inline int vis_ring(int n) {  // points in the ring
-    const int w = vis_chunk(n) + 3;
+__host__ __device__ inline int vis_ring(int n, int cmax) {  // points in the ring
+    const int w = vis_chunk(n, cmax) + 3;
     return w < n + 4 ? w : n + 4;
 }
 // lanes of a row of the ring: odd for i-lines, whose loads walk along a line
@@ -153,12 +153,12 @@ __device__ __forceinline__ void copy8_async(double *dst, const double *src) {
 // out[m*stride + point] for an ordered combine (k_combine_dq).
 template <int dir>
 __global__ void __launch_bounds__(VIS_THREADS, VIS_CTAS) k_rhs_vis(DevParams P, DevFields F, const DevBlock *__restrict__ blocks,
-                                                    const LineGroup *__restrict__ groups, double *out, long long stride) {
+                                                    const LineGroup *__restrict__ groups, int cmax, double *out, long long stride) {
     extern __shared__ __align__(16) double smem[];
     const LineGroup G = groups[blockIdx.x];
     const DevBlock B = blocks[G.blk];
     const int n = dimof(B, dir), NL = G.nl, NLP = vis_row(dir, NL);
-    const int H = n + 1, C = vis_chunk(n), RP = vis_ring(n), FR = C + 5;
+    const int H = n + 1, C = vis_chunk(n, cmax), RP = vis_ring(n, cmax), FR = C + 5;
     double *fv = smem + RP * NLP * VIS_PITCH;  // the last FR half nodes' fluxes
     __shared__ int flags[VIS_MAX_LINES];       // bit 0: the left end has a boundary, bit 1: the right end
     constexpr int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
@@ -378,19 +378,20 @@ __global__ void __launch_bounds__(VIS_THREADS, VIS_CTAS) k_rhs_vis(DevParams P, 
     }
 }
 
-size_t rhs_vis_line_bytes(int dir, int n, int nl) {
-    return sizeof(double) * (size_t)vis_row(dir, nl) * (vis_ring(n) * VIS_PITCH + VIS_FP * (vis_chunk(n) + 5));
+size_t rhs_vis_line_bytes(int dir, int n, int nl, int cmax) {
+    return sizeof(double) * (size_t)vis_row(dir, nl) * (vis_ring(n, cmax) * VIS_PITCH + VIS_FP * (vis_chunk(n, cmax) + 5));
 }
-int rhs_vis_lines(int n) { return std::min(VIS_MAX_LINES, VIS_THREADS / vis_chunk(n)); }
+int rhs_vis_lines(int n, int cmax) { return std::min(VIS_MAX_LINES, VIS_THREADS / vis_chunk(n, cmax)); }
+int rhs_vis_chunks(int n, int cmax) { return (n + vis_chunk(n, cmax)) / vis_chunk(n, cmax); }
 
 void launch_rhs_vis(const LaunchCtx &c, int dir, cudaStream_t st, double *out) {
     if (c.mixed) return launch_rhs_vis_mx(c, dir, st, out);
     const DirTable &T = c.vis[dir];
     if (T.ngroups == 0) return;
     const long long stride = c.total;
-    if (dir == 0) k_rhs_vis<0><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, out, stride);
-    else if (dir == 1) k_rhs_vis<1><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, out, stride);
-    else k_rhs_vis<2><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, out, stride);
+    if (dir == 0) k_rhs_vis<0><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.cmax, out, stride);
+    else if (dir == 1) k_rhs_vis<1><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.cmax, out, stride);
+    else k_rhs_vis<2><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.cmax, out, stride);
 }
 
 void setup_rhs_vis_attrs(size_t max_smem) {

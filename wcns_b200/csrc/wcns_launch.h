@@ -15,7 +15,7 @@ struct LineGroup {
 
 struct DirTable {
     LineGroup *groups = nullptr;  // device
-    int ngroups = 0;
+    int ngroups = 0, cmax = 0;  // cmax: half nodes per chunk at most, in the FP64 line kernels
     size_t smem = 0;              // dynamic shared memory of the launch (max over groups)
 };
 
@@ -239,17 +239,19 @@ inline void launch_block_clusters(void (*kern)(KArgs...), int nblocks, int threa
 
 void launch_rhs_invis(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
 void setup_rhs_invis_attrs(size_t max_smem, int nflux);
-size_t rhs_invis_line_bytes(int n, bool sections);  // shared memory of one line in k_rhs_invis
-int rhs_invis_threads();             // threads per CTA in k_rhs_invis
-size_t rhs_invis_smem();             // staged lines per CTA at most, bytes
-int rhs_invis_max_lines();           // lines per CTA in k_rhs_invis
+// shared memory of nl lines, lines per CTA and chunks per line in the FP64 line
+// kernels with chunks of at most cmax half nodes
+size_t rhs_invis_line_bytes(int dir, int n, int nl, int cmax, bool sections);
+int rhs_invis_lines(int n, int cmax);
+int rhs_invis_chunks(int n, int cmax);
+size_t rhs_vis_line_bytes(int dir, int n, int nl, int cmax);
+int rhs_vis_lines(int n, int cmax);
+int rhs_vis_chunks(int n, int cmax);
 void launch_node_derivatives(const LaunchCtx &c);
 void launch_rhs_vis(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
 // all three directions of the viscous (vis = true) or inviscid residual
 void launch_rhs_dirs(const LaunchCtx &c, bool vis);
 void setup_rhs_vis_attrs(size_t max_smem);
-size_t rhs_vis_line_bytes(int dir, int n, int nl);  // shared memory of nl lines in k_rhs_vis
-int rhs_vis_lines(int n);                           // lines per CTA in k_rhs_vis
 size_t adj_line_bytes(int n);     // shared memory of one line in the adjoint's kernels
 int adj_max_lines();              // lines per CTA in the adjoint's kernels
 constexpr int ADJ_REC_WORDS = 52; // doubles per cell of the LU-SGS operator's records
