@@ -16,6 +16,10 @@ pytestmark = pytest.mark.gpu
 
 DQ = ["dq1", "dq2", "dq3", "dq4", "dq5"]
 DIMS = [(5, 6, 7), (7, 5, 8), (8, 9, 10), (12, 11, 5), (31, 8, 33), (10, 64, 6), (6, 13, 65), (71, 9, 11), (130, 7, 6), (9, 6, 257)]
+# enough lines for the shortest chunks: lengths whose first chunk takes every remainder
+LARGE = [(90 + q % 5, 96 + q, 92 + q % 3) for q in range(8)]
+INVISCID = [(d, s, f) for d in DIMS for s in (4, 41, 42) for f in (1, 2, 3)] + \
+    [(d, (4, 41, 42)[q % 3], (3, 2, 1)[q % 3 if q < 3 else 0]) for q, d in enumerate(LARGE)] + [(d, 41, 3) for d in LARGE]
 
 
 def _case(dims, nscheme, nflux):
@@ -32,9 +36,7 @@ def _case(dims, nscheme, nflux):
     return case
 
 
-@pytest.mark.parametrize("nflux", [1, 2, 3])
-@pytest.mark.parametrize("nscheme", [4, 41, 42])
-@pytest.mark.parametrize("dims", DIMS, ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("dims,nscheme,nflux", INVISCID, ids=str)
 def test_inviscid_lines(dims, nscheme, nflux):
     from oracle.pyoracle import Oracle
     from wcns_b200.solver import Wcns
@@ -47,7 +49,7 @@ def test_inviscid_lines(dims, nscheme, nflux):
     assert max(errs.values()) <= 1e-12, errs
 
 
-@pytest.mark.parametrize("dims", DIMS + [(4, 6, 7), (9, 5, 3), (6, 4, 5)], ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("dims", DIMS + LARGE + [(4, 6, 7), (9, 5, 3), (6, 4, 5)], ids=lambda d: "x".join(map(str, d)))
 def test_viscous_lines(dims):
     from oracle.pyoracle import Oracle
     from wcns_b200.solver import Wcns
