@@ -502,6 +502,14 @@ static int build_tables(WcnsContext *c) {
         }
     }
     first[nbk] = (int)regs.size();
+    int region_pts = 1;
+    for (const DevRegion &d : regs) region_pts = std::max(region_pts, (d.s_ed[0] - d.s_st[0] + 1) * (d.s_ed[1] - d.s_st[1] + 1) * (d.s_ed[2] - d.s_st[2] + 1));
+    // the largest region in one pass of the block's cluster, but no more threads than
+    // let all clusters run at once (16 warps of 112 registers per SM): 64 small blocks 248 us at
+    // 512 threads, 104 at one pass (160), 64 at 128; the channel's 24 blocks 112 us at
+    // 512 and 98 at 256; six blocks 51 us at 512, 60 at 256
+    L.bc_threads = std::min(BC_MAX_THREADS, std::max(64, (region_pts + 32 * BC_CLUSTER - 1) / (32 * BC_CLUSTER) * 32));
+    while (L.bc_threads > 64 && nbk * BC_CLUSTER > 148 * (512 / L.bc_threads)) L.bc_threads -= 32;
     L.regions = c->up(regs);
     L.reg_first = c->up(first);
     L.nsa_if = (long long)sa_src.size();

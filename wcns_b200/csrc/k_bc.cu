@@ -34,8 +34,11 @@ __global__ void k_ghost_copy(DevFields F, const GhostCopy *__restrict__ list, lo
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
         GhostCopy g = list[e];
+        double v[5];  // all loads before the first store, which they may not pass
 #pragma unroll
-        for (int f = 0; f < 5; f++) F.f[F_R + f][g.dst] = F.f[F_R + f][g.src];
+        for (int f = 0; f < 5; f++) v[f] = F.f[F_R + f][g.src];
+#pragma unroll
+        for (int f = 0; f < 5; f++) F.f[F_R + f][g.dst] = v[f];
     }
     if (qke)
         for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nsa; e += stride) {
@@ -52,6 +55,23 @@ __device__ __forceinline__ void set5(DevFields &F, long long id, double r, doubl
     F.f[F_W][id] = w;
     F.f[F_P][id] = p;
 }
+
+// the three points inside a face point: all loads at once, before the ghosts' stores,
+// which they may not pass (a region took five dependent trips to L2 per ghost layer)
+struct Mirror {
+    double r[3], u[3], v[3], w[3], p[3];
+    __device__ __forceinline__ void load(const DevFields &F, long long f, long long sL) {
+#pragma unroll
+        for (int l = 0; l < 3; l++) {
+            const long long t = f - (l + 1) * sL;
+            r[l] = F.f[F_R][t];
+            u[l] = F.f[F_U][t];
+            v[l] = F.f[F_V][t];
+            w[l] = F.f[F_W][t];
+            p[l] = F.f[F_P][t];
+        }
+    }
+};
 
 // getnxyz_mml (Sub1.f90:750-780)
 __device__ __forceinline__ void getnxyz(const DevFields &F, long long id, int is, int js, int ks, double &nx, double &ny,
@@ -86,7 +106,7 @@ __device__ __forceinline__ void getnxyz(const DevFields &F, long long id, int is
 // Interface regions come first in a block's list (set_bc_index), so a point
 // that two regions share keeps the later region's value, as in the
 // reference's sequence.
-__global__ void __launch_bounds__(512) k_bc_physical(DevParams P, DevFields F, const DevBlock *__restrict__ blocks,
+__global__ void __launch_bounds__(BC_MAX_THREADS) k_bc_physical(DevParams P, DevFields F, const DevBlock *__restrict__ blocks,
                                                      const DevRegion *__restrict__ regions,
                                                      const int *__restrict__ reg_first, double *__restrict__ qke,
                                                      const long long *__restrict__ sa_src,
@@ -194,40 +214,51 @@ __global__ void __launch_bounds__(512) k_bc_physical(DevParams P, DevFields F, c
             }
             case 2: {
                 if (P.nvis == 1) {  // viscous wall
-                    long long t1 = f - sL, t2 = f - 2 * sL, t3 = f - 3 * sL;
-                    set5(F, f + sL, rr[t1], -uu[t1], -vv[t1], -ww[t1], pp[t1]);
-                    if (qke) {
-                        qke[f + sL] = -qke[t1];
-                        qke[f] = 0.5 * (qke[t1] + qke[f + sL]);
+                    Mirror M;
+                    M.load(F, f, sL);
+                    const double q1 = qke ? qke[f - sL] : 0.0;
+                    double t1 = 0.0, t2 = 0.0;
+                    if (P.adiabatic) {
+                        t1 = F.f[F_T][f - sL];
+                        t2 = F.f[F_T][f - 2 * sL];
                     }
-                    double pres = (4.0 * pp[t1] - pp[t2]) / 3.0;
+                    set5(F, f + sL, M.r[0], -M.u[0], -M.v[0], -M.w[0], M.p[0]);
+                    if (qke) {
+                        qke[f + sL] = -q1;
+                        qke[f] = 0.5 * (q1 + -q1);
+                    }
+                    double pres = (4.0 * M.p[0] - M.p[1]) / 3.0;
                     double tres;
                     if (P.adiabatic) {
-                        const double *tt = F.f[F_T];
-                        tres = (4.0 * tt[t1] - tt[t2]) / 3.0;
-                        if (pres < PMIN_LIMIT) pres = pp[t1];
-                        if (tres < TMIN_LIMIT) tres = tt[t1];
+                        tres = (4.0 * t1 - t2) / 3.0;
+                        if (pres < PMIN_LIMIT) pres = M.p[0];
+                        if (tres < TMIN_LIMIT) tres = t1;
                     } else {
-                        if (pres < PMIN_LIMIT) pres = pp[t1];
+                        if (pres < PMIN_LIMIT) pres = M.p[0];
                         tres = P.twall_nd;
                     }
                     double dres = B.moocp * pres / tres;
                     set5(F, f, dres, 0.0, 0.0, 0.0, pres);
-                    set5(F, f + 2 * sL, rr[t2], -uu[t2], -vv[t2], -ww[t2], pp[t2]);
-                    set5(F, f + 3 * sL, -rr[t3], -uu[t3], -vv[t3], -ww[t3], pp[t3]);
+                    set5(F, f + 2 * sL, M.r[1], -M.u[1], -M.v[1], -M.w[1], M.p[1]);
+                    set5(F, f + 3 * sL, -M.r[2], -M.u[2], -M.v[2], -M.w[2], M.p[2]);
                 } else {  // inviscid wall + dif_average
                     double nx, ny, nz;
                     getnxyz(F, f, L[0], L[1], L[2], nx, ny, nz);
+                    Mirror M;
+                    M.load(F, f, sL);
+                    const double q1 = qke ? qke[f - sL] : 0.0, qg = qke ? qke[f + sL] : 0.0;
+                    double g[5];  // the first ghost
+#pragma unroll
                     for (int l = 1; l <= 3; l++) {
-                        long long s = f + l * sL, tI = f - l * sL;
-                        double s1 = 2.0 * (uu[tI] * nx + vv[tI] * ny + ww[tI] * nz);
-                        double rv = l == 3 ? -rr[tI] : rr[tI];
-                        set5(F, s, rv, uu[tI] - s1 * nx, vv[tI] - s1 * ny, ww[tI] - s1 * nz, pp[tI]);
+                        double s1 = 2.0 * (M.u[l - 1] * nx + M.v[l - 1] * ny + M.w[l - 1] * nz);
+                        double rv = l == 3 ? -M.r[l - 1] : M.r[l - 1];
+                        const double gu = M.u[l - 1] - s1 * nx, gv = M.v[l - 1] - s1 * ny, gw = M.w[l - 1] - s1 * nz;
+                        if (l == 1) { g[0] = rv; g[1] = gu; g[2] = gv; g[3] = gw; g[4] = M.p[0]; }
+                        set5(F, f + l * sL, rv, gu, gv, gw, M.p[l - 1]);
                     }
-                    long long s = f + sL, tI = f - sL;
-                    set5(F, f, 0.5 * (rr[s] + rr[tI]), 0.5 * (uu[s] + uu[tI]), 0.5 * (vv[s] + vv[tI]), 0.5 * (ww[s] + ww[tI]),
-                         0.5 * (pp[s] + pp[tI]));
-                    if (qke) qke[f] = 0.5 * (qke[tI] + qke[s]);
+                    set5(F, f, 0.5 * (g[0] + M.r[0]), 0.5 * (g[1] + M.u[0]), 0.5 * (g[2] + M.v[0]), 0.5 * (g[3] + M.w[0]),
+                         0.5 * (g[4] + M.p[0]));
+                    if (qke) qke[f] = 0.5 * (q1 + qg);
                 }
                 break;
             }
@@ -243,18 +274,29 @@ __global__ void __launch_bounds__(512) k_bc_physical(DevParams P, DevFields F, c
                     set5(F, f + sL, rm, um, vm, wm, pm);
                     set5(F, f + 2 * sL, rm, um, vm, 0.0, pm);
                     set5(F, f + 3 * sL, rm, um, vm, 0.0, pm);
+                    long long s = f + sL, t1 = f - sL;
+                    set5(F, f, 0.5 * (rr[s] + rr[t1]), 0.5 * (uu[s] + uu[t1]), 0.5 * (vv[s] + vv[t1]), 0.5 * (ww[s] + ww[t1]),
+                         0.5 * (pp[s] + pp[t1]));
+                    if (qke) qke[f] = 0.5 * (qke[t1] + qke[s]);
                 } else {
+                    Mirror M;
+                    M.load(F, f, sL);
+                    const double q1 = qke ? qke[f - sL] : 0.0;
+                    double g[5];  // the first ghost
+#pragma unroll
                     for (int l = 1; l <= 3; l++) {
-                        long long s = f + l * sL, tI = f - l * sL;
-                        double s1 = 2.0 * (snx * uu[tI] + sny * vv[tI] + snz * ww[tI]);
-                        set5(F, s, rr[tI], uu[tI] - s1 * snx, vv[tI] - s1 * sny, ww[tI] - s1 * snz, pp[tI]);
-                        if (l == 1 && qke) qke[s] = qke[tI];
+                        double s1 = 2.0 * (snx * M.u[l - 1] + sny * M.v[l - 1] + snz * M.w[l - 1]);
+                        const double gu = M.u[l - 1] - s1 * snx, gv = M.v[l - 1] - s1 * sny, gw = M.w[l - 1] - s1 * snz;
+                        if (l == 1) { g[0] = M.r[0]; g[1] = gu; g[2] = gv; g[3] = gw; g[4] = M.p[0]; }
+                        set5(F, f + l * sL, M.r[l - 1], gu, gv, gw, M.p[l - 1]);
+                    }
+                    set5(F, f, 0.5 * (g[0] + M.r[0]), 0.5 * (g[1] + M.u[0]), 0.5 * (g[2] + M.v[0]), 0.5 * (g[3] + M.w[0]),
+                         0.5 * (g[4] + M.p[0]));
+                    if (qke) {
+                        qke[f + sL] = q1;
+                        qke[f] = 0.5 * (q1 + q1);
                     }
                 }
-                long long s = f + sL, tI = f - sL;
-                set5(F, f, 0.5 * (rr[s] + rr[tI]), 0.5 * (uu[s] + uu[tI]), 0.5 * (vv[s] + vv[tI]), 0.5 * (ww[s] + ww[tI]),
-                     0.5 * (pp[s] + pp[tI]));
-                if (qke) qke[f] = 0.5 * (qke[tI] + qke[s]);
                 break;
             }
             case -1: {  // interface: the SA model's qke/vist copy and face mean
@@ -262,10 +304,11 @@ __global__ void __launch_bounds__(512) k_bc_physical(DevParams P, DevFields F, c
                 double pv, pq;
                 if (R.same) { pq = qke[sa_src[e]]; pv = vist[sa_src[e]]; }
                 else { pq = sa_snap[2 * e]; pv = sa_snap[2 * e + 1]; }
+                const double vi = vist[tI], qi = qke[tI];
                 vist[g] = pv;
-                vist[f] = (vist[g] + vist[tI]) * 0.5;
+                vist[f] = (pv + vi) * 0.5;
                 qke[g] = pq;
-                qke[f] = (qke[g] + qke[tI]) * 0.5;
+                qke[f] = (pq + qi) * 0.5;
                 break;
             }
             default: break;
@@ -283,7 +326,7 @@ void launch_boundary(const LaunchCtx &c) {
                                                  c.sa_if_snap, c.nsa_if);
     }
     double *qke = c.SA ? c.SA->qke : nullptr;
-    launch_block_clusters(k_bc_physical, c.nblocks, 512, c.stream, *c.P, *c.F, (const DevBlock *)c.blocks,
+    launch_block_clusters(k_bc_physical, c.nblocks, c.bc_threads, c.stream, *c.P, *c.F, (const DevBlock *)c.blocks,
                           (const DevRegion *)c.regions, (const int *)c.reg_first, qke, (const long long *)c.sa_if_src,
                           (const double *)c.sa_if_snap);
 }

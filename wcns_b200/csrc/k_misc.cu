@@ -417,12 +417,17 @@ __global__ void k_snapshot(DevFields F, const long long *__restrict__ pts, int n
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         long long id = pts[s];
         if (which == 0) {
-            double vol = F.f[F_VOL][id];
+            double vol = F.f[F_VOL][id], v[5];  // all loads before the first store, which they may not pass
 #pragma unroll
-            for (int m = 0; m < 5; m++) snap[(long long)m * n + s] = F.f[F_DQ1 + m][id] / vol;
+            for (int m = 0; m < 5; m++) v[m] = F.f[F_DQ1 + m][id];
+#pragma unroll
+            for (int m = 0; m < 5; m++) snap[(long long)m * n + s] = v[m] / vol;
         } else {
+            double v[6];
 #pragma unroll
-            for (int m = 0; m < 6; m++) snap[(long long)m * n + s] = F.f[F_R + m][id];
+            for (int m = 0; m < 6; m++) v[m] = F.f[F_R + m][id];
+#pragma unroll
+            for (int m = 0; m < 6; m++) snap[(long long)m * n + s] = v[m];
         }
     }
 }
@@ -446,29 +451,29 @@ __global__ void k_match(DevFields F, const PairEntry *__restrict__ pairs, const 
     for (int r = blk_reg_first[bi]; r < blk_reg_first[bi + 1]; r++) {
         for (int e = reg_pair_first[r] + t0; e < reg_pair_first[r + 1]; e += tstride) {
             PairEntry pe = pairs[e];
+            // all loads of a pair before its first store, which they may not pass: a trip
+            // to L2 per pair, not one per component (both exchanges of a step on a
+            // vortex of 65x33x17 points 66 -> 49 us)
+            double own[6], oth[6];
             if (which == 0) {
                 double vs = F.f[F_VOL][pe.own];
-                if (pe.same) {
-                    double vol_p = vs / F.f[F_VOL][pe.partner];
+                const double vp = pe.same ? F.f[F_VOL][pe.partner] : 1.0;
 #pragma unroll
-                    for (int m = 0; m < 5; m++) {
-                        double *dq = F.f[F_DQ1 + m];
-                        dq[pe.own] = 0.5 * (dq[pe.partner] * vol_p + dq[pe.own]);
-                    }
-                } else {
-#pragma unroll
-                    for (int m = 0; m < 5; m++) {
-                        double *dq = F.f[F_DQ1 + m];
-                        dq[pe.own] = 0.5 * (snap[(long long)m * nsnap + pe.partner_slot] * vs + dq[pe.own]);
-                    }
+                for (int m = 0; m < 5; m++) {
+                    own[m] = F.f[F_DQ1 + m][pe.own];
+                    oth[m] = pe.same ? F.f[F_DQ1 + m][pe.partner] : snap[(long long)m * nsnap + pe.partner_slot];
                 }
+                const double k = pe.same ? vs / vp : vs;
+#pragma unroll
+                for (int m = 0; m < 5; m++) F.f[F_DQ1 + m][pe.own] = 0.5 * (oth[m] * k + own[m]);
             } else {
 #pragma unroll
                 for (int m = 0; m < 6; m++) {
-                    double *x = F.f[F_R + m];
-                    double tv = pe.same ? x[pe.partner] : snap[(long long)m * nsnap + pe.partner_slot];
-                    x[pe.own] = 0.5 * (tv + x[pe.own]);
+                    own[m] = F.f[F_R + m][pe.own];
+                    oth[m] = pe.same ? F.f[F_R + m][pe.partner] : snap[(long long)m * nsnap + pe.partner_slot];
                 }
+#pragma unroll
+                for (int m = 0; m < 6; m++) F.f[F_R + m][pe.own] = 0.5 * (oth[m] + own[m]);
             }
         }
         cluster.sync();

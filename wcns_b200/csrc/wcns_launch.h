@@ -132,6 +132,7 @@ struct LaunchCtx {
     cudaStream_t side[2] = {nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
     double *contrib = nullptr;         // 2 directions x 5 components x total
+    int bc_threads = 512;              // threads per CTA in k_bc_physical: a region in one pass
     const DevParams *P = nullptr;  // host copy, passed by value
     const DevFields *F = nullptr;
     DevBlock *blocks = nullptr;    // device
@@ -219,6 +220,7 @@ inline void prof_mark(const LaunchCtx &c, const char *name) {
 // CTAs per block for the kernels that walk a block's BC or interface
 // regions in order (one cluster per block, cluster barrier between regions)
 constexpr int BC_CLUSTER = 8;
+constexpr int BC_MAX_THREADS = 512;  // threads per CTA in k_bc_physical at most (LaunchCtx::bc_threads)
 
 template <class... KArgs, class... Args>
 inline void launch_block_clusters(void (*kern)(KArgs...), int nblocks, int threads, cudaStream_t stream, Args... args) {
