@@ -140,3 +140,25 @@ def test_switch_to_wide_sweeps_and_back():
     a, ha, _, _ = _run(sa)
     b, hb, _, _ = _run(sa, [0, 0, 32, 32]) if a.shape[0] else (a, ha, None, None)
     np.testing.assert_allclose(hb, ha, rtol=1e-11, atol=0)
+
+
+@pytest.mark.gpu
+def test_cluster_size_changed_between_steps():
+    """Another cluster size lays the sweeps' slots out differently: what the last one
+    left there must not reach the next step."""
+    from tests.helpers import perturbed
+    from wcns_b200.solver import Wcns
+    out = []
+    for shapes in (((0, 0),), ((4, 0), (16, 1), (8, 0)), ((16, 1), (2, 1), (8, 1))):
+        g = Wcns(perturbed(cases.vortex_case(ni=30, nj=18, nk=11, nscheme=4, nflux=1)))
+        for q in range(3):
+            a, b = shapes[min(q, len(shapes) - 1)]
+            try:
+                g.set_shape([a, b] + list(g.shape)[2:])
+            except Exception:  # a shape that these blocks cannot run
+                pass
+            g.step(1)
+        out.append([g.get(f, 1) for f in ("r", "u", "v", "w", "p")])
+    for other in out[1:]:
+        for x, y in zip(out[0], other):
+            np.testing.assert_array_equal(x, y)

@@ -86,6 +86,7 @@ struct WcnsContext {
     long long total = 0;      // ghosted points over all blocks
     long long total_pm = 0;   // plane-major sweep points over all blocks
     double *pool = nullptr;
+    size_t pm_bytes = 0;
     double *pm_pool = nullptr;
     PmFields PM{};
     cudaStream_t stream = nullptr;
@@ -318,12 +319,22 @@ static int pm_alloc(WcnsContext *c) {
         return WCNS_ERR_CUDA;
     }
     CK(cudaMemset(c->pm_pool, 0, pmbytes));
+    c->pm_bytes = pmbytes;
     for (int m = 0; m < 5; m++) c->PM.dq[m] = c->pm_pool + (size_t)m * c->total_pm;
     c->PM.dq_stride = c->total_pm;
     c->PM.stat = c->pm_pool + (size_t)5 * c->total_pm;
     c->PM.dyn = c->PM.stat + (size_t)SR_N * c->total_pm;
     c->PM.gs[0] = c->PM.dyn + (size_t)DYN_N * c->total_pm;
     c->PM.gs[1] = c->PM.gs[0] + (size_t)DYN_N * c->total_pm;
+    return 0;
+}
+
+// The sweeps' slots for clusters of csize CTAs.  They never write the slots outside
+// the block, which stay zero; another cluster size lays the slots out differently and
+// leaves its values there.
+static int pm_layout(WcnsContext *c, int csize) {
+    if (c->pm_pool && c->PM.csize != csize) CK(cudaMemsetAsync(c->pm_pool, 0, c->pm_bytes, c->stream));
+    c->PM.csize = csize;
     return 0;
 }
 
@@ -1661,7 +1672,7 @@ static int apply_shape(WcnsContext *c, const int *shape) {
                 return WCNS_ERR_ARGUMENT;
             }
             if (int rc = pm_alloc(c)) return rc;
-            c->PM.csize = L.sweep_cluster;
+            if (int rc = pm_layout(c, L.sweep_cluster)) return rc;
             wide_free(c);
         }
     }
@@ -1740,7 +1751,7 @@ extern "C" int wcns_autotune(WcnsContext *c, int reps, int *shape, double *ms) {
             for (int q = 0; q < 5; q++) {
                 int cand[4] = {cls[q], fine, best[2], best[3]};
                 if (setup_sweep_exact(L, cand[0], cand[1])) continue;
-                c->PM.csize = L.sweep_cluster;
+                if (int rc = pm_layout(c, L.sweep_cluster)) { cudaFree(saved); return rc; }
                 const double t = time_reps(c, reps, saved, [&] { launch_lhs(L); });
                 if (t < tbest) { tbest = t; best[0] = cand[0]; best[1] = cand[1]; }
             }
@@ -1753,7 +1764,7 @@ extern "C" int wcns_autotune(WcnsContext *c, int reps, int *shape, double *ms) {
         }
         if (best[0] > 0) {
             setup_sweep_exact(L, best[0], best[1]);
-            c->PM.csize = L.sweep_cluster;
+            if (int rc = pm_layout(c, L.sweep_cluster)) return rc;
             wide_free(c);
         }
         best_ms[0] = tbest;

@@ -858,8 +858,8 @@ int setup_sweep_wide(LaunchCtx &c, WideSweep &W) {
         per_sm = std::min(per_sm, q);
     };
     for (int m = 0; m < 4; m++) fits(pick[m].fn, pick[m].smem);
-    cudaFuncSetAttribute(k_sa_sweep_wide<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sa_smem(threads, nkmax));
-    cudaFuncSetAttribute(k_sa_sweep_wide<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sa_smem(threads, nkmax));
+    cudaFuncSetAttribute(k_sa_sweep_wide<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM);
+    cudaFuncSetAttribute(k_sa_sweep_wide<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM);
     fits(k_sa_sweep_wide<true>, sa_smem(threads, nkmax));
     fits(k_sa_sweep_wide<false>, sa_smem(threads, nkmax));
     if (verbose)
