@@ -444,10 +444,10 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
         }
     }
     if (inv_smem > 227 * 1024 || vis_smem > 227 * 1024) { set_err("line too long for shared memory"); return WCNS_ERR_ARGUMENT; }
-    setup_rhs_invis_attrs(std::max<size_t>(inv_smem, 48 * 1024), c->P.nflux);
-    setup_rhs_vis_attrs(std::max<size_t>(vis_smem, 48 * 1024));
+    setup_rhs_invis_attrs(c->P.nflux);
+    setup_rhs_vis_attrs();
     if (inv_mx_smem > 227 * 1024 || vis_mx_smem > 227 * 1024) { set_err("line too long for shared memory"); return WCNS_ERR_ARGUMENT; }
-    setup_rhs_mx_attrs(std::max<size_t>(inv_mx_smem, 48 * 1024), std::max<size_t>(vis_mx_smem, 48 * 1024));
+    setup_rhs_mx_attrs();
     L.inv_cap = inv_cap;
     L.vis_cap = vis_cap;
     return 0;
@@ -1810,6 +1810,7 @@ static int adj_ready(WcnsContext *c, const char *who) {
         return WCNS_ERR_UNSUPPORTED;
     }
     if (!c->adj_pool) {
+        setup_adj_attrs();
         const size_t bytes = sizeof(double) * 5 * (size_t)WCNS_ADJ_NSLOTS * (size_t)c->total;
         CK(cudaMalloc(&c->adj_pool, bytes));
         CK(cudaMemset(c->adj_pool, 0, bytes));

@@ -922,6 +922,14 @@ __global__ void k_adj_reduce(const DevBlock *__restrict__ blocks, double *y, con
 // ---------------------------------------------------------------------------
 // launches
 // ---------------------------------------------------------------------------
+void setup_adj_attrs() {
+    allow_all_smem(k_rhs_invis_jvp<0>);
+    allow_all_smem(k_rhs_invis_jvp<1>);
+    allow_all_smem(k_rhs_invis_jvp<2>);
+    allow_all_smem(k_rhs_invis_vjp<0>);
+    allow_all_smem(k_rhs_invis_vjp<1>);
+    allow_all_smem(k_rhs_invis_vjp<2>);
+}
 size_t adj_line_bytes(int n) { return (size_t)adj_line_stride(n) * sizeof(double); }
 int adj_max_lines() { return INV_LINES_DEFAULT; }
 
@@ -931,13 +939,10 @@ void launch_rhs_invis_jvp(const LaunchCtx &c, const double *v, double *out) {
         if (!T.ngroups) continue;
         const size_t sm = T.smem;
         if (d == 0) {
-            cudaFuncSetAttribute(k_rhs_invis_jvp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_rhs_invis_jvp<0><<<T.ngroups, 256, sm, c.stream>>>(*c.P, *c.F, c.blocks, T.groups, v, out, c.total);
         } else if (d == 1) {
-            cudaFuncSetAttribute(k_rhs_invis_jvp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_rhs_invis_jvp<1><<<T.ngroups, 256, sm, c.stream>>>(*c.P, *c.F, c.blocks, T.groups, v, out, c.total);
         } else {
-            cudaFuncSetAttribute(k_rhs_invis_jvp<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_rhs_invis_jvp<2><<<T.ngroups, 256, sm, c.stream>>>(*c.P, *c.F, c.blocks, T.groups, v, out, c.total);
         }
     }
@@ -949,13 +954,10 @@ void launch_rhs_invis_vjp(const LaunchCtx &c, const double *lam, double *out, bo
         if (!T.ngroups) continue;
         const size_t sm = T.smem;
         if (d == 0) {
-            cudaFuncSetAttribute(k_rhs_invis_vjp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_rhs_invis_vjp<0><<<T.ngroups, 256, sm, c.stream>>>(*c.P, *c.F, c.blocks, T.groups, lam, out, c.total);
         } else if (d == 1) {
-            cudaFuncSetAttribute(k_rhs_invis_vjp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_rhs_invis_vjp<1><<<T.ngroups, 256, sm, c.stream>>>(*c.P, *c.F, c.blocks, T.groups, lam, out, c.total);
         } else {
-            cudaFuncSetAttribute(k_rhs_invis_vjp<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             k_rhs_invis_vjp<2><<<T.ngroups, 256, sm, c.stream>>>(*c.P, *c.F, c.blocks, T.groups, lam, out, c.total);
         }
     }

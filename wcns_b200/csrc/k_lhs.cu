@@ -546,9 +546,9 @@ static void launch_sweep(const LaunchCtx &c) {
 }
 
 template <bool FINE>
-static void sweep_attrs(int smem, bool nonportable) {
+static void sweep_attrs(bool nonportable) {
     auto set = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        allow_all_smem(kern);
         if (nonportable) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     };
     set(k_sweep<0, FINE>);
@@ -568,7 +568,7 @@ static bool try_sweep_shape(LaunchCtx &c, int cl, int cpc) {
     const int lanes = FINE ? 16 : 3, maxt = FINE ? SWEEP_FINE_MAX_THREADS : SWEEP_COARSE_MAX_THREADS;
     const int threads = (lanes * cpc + 31) / 32 * 32 + 32;  // compute warps + the control warp
     if (threads > maxt || sm > 200 * 1024) return false;
-    sweep_attrs<FINE>((int)sm, cl > 8);
+    sweep_attrs<FINE>(cl > 8);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3(c.nblocks * cl, 1, 1);
@@ -621,12 +621,7 @@ int setup_sweep_exact(LaunchCtx &c, int cl, int fine) {
     }
     if (cl < 1 || cl > 16 || cl > minnj) return -1;
     const int cpc = (maxnj + cl - 1) / cl * maxnk;
-    const int old_cl = c.sweep_cluster, old_cpc = c.sweep_cpc, old_fine = c.sweep_fine;
-    if (fine ? try_sweep_shape<true>(c, cl, cpc) : try_sweep_shape<false>(c, cl, cpc)) return 0;
-    // a refused shape may have changed the kernels' shared-memory attributes
-    if (old_fine) try_sweep_shape<true>(c, old_cl, old_cpc);
-    else try_sweep_shape<false>(c, old_cl, old_cpc);
-    return -1;
+    return (fine ? try_sweep_shape<true>(c, cl, cpc) : try_sweep_shape<false>(c, cl, cpc)) ? 0 : -1;
 }
 
 int launch_lhs(const LaunchCtx &c) {

@@ -374,7 +374,7 @@ void launch_rhs_dirs(const LaunchCtx &c, bool vis) {
 int setup_residual(int nblocks, int ctas) {
     const size_t bytes = sizeof(double) * 2 * (size_t)nblocks * ctas;
     if (bytes > 200 * 1024) return -1;
-    if (bytes > 48 * 1024) cudaFuncSetAttribute(k_residual_final, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    allow_all_smem(k_residual_final);
     return 0;
 }
 

@@ -408,16 +408,16 @@ void launch_rhs_invis(const LaunchCtx &c, int dir, cudaStream_t st, double *out)
 }
 
 template <int NFLUX>
-static void set_invis_attrs(int max_smem) {
-    cudaFuncSetAttribute(k_rhs_invis<0, NFLUX>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(k_rhs_invis<1, NFLUX>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(k_rhs_invis<2, NFLUX>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+static void set_invis_attrs() {
+    allow_all_smem(k_rhs_invis<0, NFLUX>);
+    allow_all_smem(k_rhs_invis<1, NFLUX>);
+    allow_all_smem(k_rhs_invis<2, NFLUX>);
 }
 
-void setup_rhs_invis_attrs(size_t max_smem, int nflux) {
-    if (nflux == 1) set_invis_attrs<1>((int)max_smem);
-    else if (nflux == 2) set_invis_attrs<2>((int)max_smem);
-    else set_invis_attrs<3>((int)max_smem);
+void setup_rhs_invis_attrs(int nflux) {
+    if (nflux == 1) set_invis_attrs<1>();
+    else if (nflux == 2) set_invis_attrs<2>();
+    else set_invis_attrs<3>();
 }
 
 size_t rhs_invis_line_bytes(int dir, int n, int nl, int cmax, bool sections) {

@@ -882,13 +882,13 @@ size_t rhs_vis_mx_line_bytes(int n) { return (size_t)mxv_line_floats(n) * 4 + (s
 int rhs_invis_mx_max_lines() { return MXI_MAX_LINES; }
 int rhs_vis_mx_max_lines() { return MXV_MAX_LINES; }
 
-void setup_rhs_mx_attrs(size_t inv_smem, size_t vis_smem) {
-    cudaFuncSetAttribute(k_rhs_invis_mx<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem);
-    cudaFuncSetAttribute(k_rhs_invis_mx<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem);
-    cudaFuncSetAttribute(k_rhs_invis_mx<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem);
-    cudaFuncSetAttribute(k_rhs_vis_mx<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vis_smem);
-    cudaFuncSetAttribute(k_rhs_vis_mx<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vis_smem);
-    cudaFuncSetAttribute(k_rhs_vis_mx<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vis_smem);
+void setup_rhs_mx_attrs() {
+    allow_all_smem(k_rhs_invis_mx<0>);
+    allow_all_smem(k_rhs_invis_mx<1>);
+    allow_all_smem(k_rhs_invis_mx<2>);
+    allow_all_smem(k_rhs_vis_mx<0>);
+    allow_all_smem(k_rhs_vis_mx<1>);
+    allow_all_smem(k_rhs_vis_mx<2>);
 }
 
 void launch_rhs_invis_mx(const LaunchCtx &c, int dir, cudaStream_t st, double *out) {

@@ -394,10 +394,10 @@ void launch_rhs_vis(const LaunchCtx &c, int dir, cudaStream_t st, double *out) {
     else k_rhs_vis<2><<<T.ngroups, VIS_THREADS, T.smem, st>>>(*c.P, *c.F, c.blocks, T.groups, T.cmax, out, stride);
 }
 
-void setup_rhs_vis_attrs(size_t max_smem) {
-    cudaFuncSetAttribute(k_rhs_vis<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
-    cudaFuncSetAttribute(k_rhs_vis<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
-    cudaFuncSetAttribute(k_rhs_vis<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
+void setup_rhs_vis_attrs() {
+    allow_all_smem(k_rhs_vis<0>);
+    allow_all_smem(k_rhs_vis<1>);
+    allow_all_smem(k_rhs_vis<2>);
 }
 
 }  // namespace wcns

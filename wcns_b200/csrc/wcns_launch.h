@@ -217,6 +217,19 @@ inline void prof_mark(const LaunchCtx &c, const char *name) {
     c.prof->name[c.prof->n++] = name;
 }
 
+// The limit of a kernel's dynamic shared memory belongs to the process and not to a
+// context: a kernel that may take more than the 48 KB every kernel has is given all
+// that the device leaves it, whatever the context at hand needs, so that no context
+// takes from another what that one launches with.
+template <class... KArgs>
+inline void allow_all_smem(void (*kern)(KArgs...)) {
+    int dev = 0, top = 0;
+    cudaFuncAttributes a = {};
+    if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&top, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) || cudaFuncGetAttributes(&a, kern)) return;
+    const int most = top - (int)a.sharedSizeBytes;
+    if (a.maxDynamicSharedSizeBytes < most) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // CTAs per block for the kernels that walk a block's BC or interface
 // regions in order (one cluster per block, cluster barrier between regions)
 constexpr int BC_CLUSTER = 8;
@@ -240,7 +253,7 @@ inline void launch_block_clusters(void (*kern)(KArgs...), int nblocks, int threa
 }
 
 void launch_rhs_invis(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
-void setup_rhs_invis_attrs(size_t max_smem, int nflux);
+void setup_rhs_invis_attrs(int nflux);
 // shared memory of nl lines, lines per CTA and chunks per line in the FP64 line
 // kernels with chunks of at most cmax half nodes
 size_t rhs_invis_line_bytes(int dir, int n, int nl, int cmax, bool sections);
@@ -253,7 +266,8 @@ void launch_node_derivatives(const LaunchCtx &c);
 void launch_rhs_vis(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
 // all three directions of the viscous (vis = true) or inviscid residual
 void launch_rhs_dirs(const LaunchCtx &c, bool vis);
-void setup_rhs_vis_attrs(size_t max_smem);
+void setup_rhs_vis_attrs();
+void setup_adj_attrs();
 size_t adj_line_bytes(int n);     // shared memory of one line in the adjoint's kernels
 int adj_max_lines();              // lines per CTA in the adjoint's kernels
 constexpr int ADJ_REC_WORDS = 52; // doubles per cell of the LU-SGS operator's records
@@ -262,7 +276,7 @@ bool adj_lu_marches(const LaunchCtx &c);  // whether its sweeps can run on recor
 void launch_rhs_invis_mx(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
 void launch_rhs_vis_mx(const LaunchCtx &c, int dir, cudaStream_t st, double *out);
 void launch_node_derivatives_mx(const LaunchCtx &c);
-void setup_rhs_mx_attrs(size_t inv_smem, size_t vis_smem);
+void setup_rhs_mx_attrs();
 size_t rhs_invis_mx_line_bytes(int n);
 size_t rhs_vis_mx_line_bytes(int n);
 int rhs_invis_mx_max_lines();
