@@ -57,9 +57,10 @@
 // it wants has the value too, so neither side needs a fence or a flag.  Tags
 // never repeat: every launch counts its planes from a base that the prep
 // kernel moves on (A.epoch).  The ring holds A.ringn planes; every eighth
-// plane the reader publishes how far it has read and the writer checks it (a
-// power of two of at least the fold delay plus 32, so that the CTA that is
-// furthest behind can always go on).  Every wait is bounded.
+// plane the reader publishes how many entries both of its ring warps have read,
+// and the writer checks it (wcns_ring.h; a power of two of at least the fold delay
+// plus 32, so that the CTA that is furthest behind can always go on).  Every wait
+// is bounded.
 //
 // Inputs are re-laid plane-major by k_wide_prep (once per step): per cell u,
 // v, w, H, the nine metrics, the inviscid radii, coed (getcoed, 602-645),
@@ -75,6 +76,7 @@
 #include <vector>
 
 #include "wcns_launch.h"
+#include "wcns_ring.h"
 #include "wcns_sweep.cuh"
 
 namespace wcns {
@@ -99,7 +101,6 @@ __device__ __forceinline__ long long rec_at(int slot, int lane, int pairs) {
 constexpr int PREP_DS = 4;        // planes per column that neighbouring lanes of a prep kernel take
 constexpr int WIDE_GAP = 4;       // idle planes between a thread's columns: a new column's copies start in the first
 constexpr int SA_ST = 4;          // planes of the scalar sweeps' words in shared memory
-constexpr int RING_CHECK = 8;     // planes between two looks at the ring's reader
 
 // a unit: the two halves of a value, each with the tag
 struct Unit { unsigned long long lo, hi; };
@@ -351,8 +352,8 @@ __device__ __forceinline__ bool copy_warp(const CtaInfo &H, const WideArrays &A,
         if ((s & (RING_CHECK - 1)) == 0 && l == 31)
             for (int g = 0; g < nseg; g++) {
                 const int sf = s - (FWD ? g : H.C.nsegmax - 1 - g) * H.C.delay, bo = FWD ? H.hi[g] : H.lo[g];
-                if (bo < 0 || sf < 0 || sf >= np || sf + RING_CHECK <= A.ringn) continue;
-                const unsigned want = tag0 + (unsigned)(sf + RING_CHECK - A.ringn);
+                if (bo < 0 || sf < 0 || sf >= np || ring_room(sf, A.ringn) <= 0) continue;
+                const unsigned want = tag0 + (unsigned)ring_room(sf, A.ringn);
                 const long long t0 = clock64(), limit = late ? (1LL << 21) : (1LL << 31);
                 while ((int)(ld_acquire(A.flags + bo) - want) < 0)
                     if (clock64() - t0 > limit) { late = true; break; }
@@ -418,10 +419,10 @@ __device__ __forceinline__ bool ring_warp(const CtaInfo &H, const WideArrays &A,
                         if (open >> q & 1) r[q] = ld_unit(e + u0 + q * 32);
                 }
             }
-            // tell the writer how far this ring has been read
-            if (((sf + 1) & (RING_CHECK - 1)) == 0) {
+            // tell the writer how far both ring warps have read
+            if (ring_publishes(sf)) {
                 __syncwarp();
-                if (l == 0) st_release(A.flags + bi, tag0 + (unsigned)(sf + 1));
+                if (l == 0) st_release(A.flags + bi, tag0 + (unsigned)ring_read(sf));
             }
         }
     }
