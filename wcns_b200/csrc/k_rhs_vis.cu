@@ -169,12 +169,10 @@ __global__ void __launch_bounds__(VIS_THREADS, VIS_CTAS) k_rhs_vis(DevParams P, 
     o[dir] = 0;
     const int base = (int)gidx(B, o[0], o[1], o[2]);          // position 0 of the first line
     const int lstep = (int)dstride(B, a1);                    // to the next line
-    if ((int)threadIdx.x < 2 * NL) {
-        const int ln = threadIdx.x >> 1, right = threadIdx.x & 1;
-        const int g = base + ln * lstep + (right ? n + 3 : -2) * st;
-        const bool f = F.f[F_R][g] < 0.0 || F.f[F_T][g] < 0.0;
-        const int other = __shfl_xor_sync(__activemask(), (int)f, 1);
-        if (!right) flags[ln] = (f ? 1 : 0) | (other ? 2 : 0);
+    if ((int)threadIdx.x < NL) {
+        const int gl = base + threadIdx.x * lstep - 2 * st, gr = gl + (n + 5) * st;
+        const double rl = F.f[F_R][gl], tl = F.f[F_T][gl], rr = F.f[F_R][gr], tr = F.f[F_T][gr];
+        flags[threadIdx.x] = (rl < 0.0 || tl < 0.0 ? 1 : 0) | (rr < 0.0 || tr < 0.0 ? 2 : 0);
     }
     // this thread's half node and line; its point and line in the loads and stores,
     // which walk along the line for i-lines and across the lines otherwise
