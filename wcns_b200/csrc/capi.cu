@@ -40,6 +40,7 @@ void set_last_error(const std::string &msg) { g_err = msg; }  // for entry point
     do {                                                                                       \
         cudaError_t e_ = (call);                                                               \
         if (e_ != cudaSuccess) {                                                               \
+            cudaGetLastError(); /* reported here: not again by the next call that looks */     \
             set_err(std::string("CUDA error: ") + cudaGetErrorString(e_) + " at " #call);      \
             return WCNS_ERR_CUDA;                                                              \
         }                                                                                      \
@@ -71,8 +72,12 @@ template <class T>
 T *dev_upload(const std::vector<T> &v) {
     if (v.empty()) return nullptr;
     T *p = nullptr;
-    if (cudaMalloc(&p, sizeof(T) * v.size()) != cudaSuccess) return nullptr;
-    cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
+    if (cudaMalloc(&p, sizeof(T) * v.size()) != cudaSuccess ||
+        cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        if (p) cudaFree(p);
+        return nullptr;
+    }
     return p;
 }
 
@@ -92,6 +97,7 @@ struct WcnsContext {
     cudaStream_t stream = nullptr;
     LaunchCtx L;
     std::vector<void *> owned;  // device allocations to free
+    bool upload_failed = false; // a table found no device memory: nothing may be launched on it
     int *d_err = nullptr;
     double *d_hist = nullptr;
     int hist_cap = 0;
@@ -133,7 +139,15 @@ struct WcnsContext {
     T *up(const std::vector<T> &v) {
         T *p = dev_upload(v);
         if (p) owned.push_back(p);
+        else if (!v.empty()) upload_failed = true;
         return p;
+    }
+    // whether every table since the last call was uploaded
+    int uploads_done() {
+        const bool failed = upload_failed;
+        upload_failed = false;
+        if (failed) set_err("device allocation of the tables failed");
+        return failed ? WCNS_ERR_CUDA : 0;
     }
     long long gi(int nb1, int i, int j, int k) const { return gidx(blk[nb1 - 1].d, i, j, k); }
 };
@@ -299,6 +313,7 @@ static int wide_alloc(WcnsContext *c) {
     }
     W->ctas = c->up(W->hctas);
     W->segs = c->up(W->hsegs);
+    if (int rc = c->uploads_done()) return rc;
     c->wide = std::move(W);
     L.wide = c->wide.get();
     return 0;
@@ -361,7 +376,15 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
     LaunchCtx &L = c->L;
     const int nbk = (int)c->blk.size();
     const bool sections = c->P.nscheme == 41 || c->P.nscheme == 42;
-    size_t inv_smem = 0, vis_smem = 0, inv_mx_smem = 0, vis_mx_smem = 0, adj_smem = 0;
+    size_t smem[5] = {};
+    // the new tables, in the place of the present ones when all of them are there
+    struct New { DirTable *old, table; };
+    std::vector<New> news;
+    auto give_up = [&](int rc) {
+        for (New &q : news) free_owned(c, q.table.groups);
+        c->upload_failed = false;
+        return rc;
+    };
     for (int dir = 0; dir < 3; dir++) {
         for (int pass = 0; pass < 5; pass++) {  // 0 inviscid, 1 viscous, 2 and 3 the same in mixed precision, 4 the adjoint's operators
             std::vector<LineGroup> g;
@@ -404,7 +427,7 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
                 const DevBlock &D = c->blk[b].d;
                 int n = dimof(D, dir);
                 if ((pass == 0 || pass == 2 || pass == 4) && n <= NIJK2D) continue;
-                if (n > MAX_LINE) { set_err("line too long for shared memory"); return WCNS_ERR_ARGUMENT; }
+                if (n > MAX_LINE) { set_err("line too long for shared memory"); return give_up(WCNS_ERR_ARGUMENT); }
                 if (pass == 4 && (c->P.nvis != 0 || c->P.nscheme != 4)) continue;  // refused there
                 int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
                 int na = dimof(D, a1), nb2 = dimof(D, a2);
@@ -429,24 +452,24 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
                                                 : pass == 1 ? rhs_vis_line_bytes(dir, n, lg.nl, cmax) : per_line * lg.nl);
                     }
             }
-            DirTable &T = pass == 0 ? L.inv[dir] : pass == 1 ? L.vis[dir] : pass == 2 ? L.inv_mx[dir] : pass == 3 ? L.vis_mx[dir] : L.adj[dir];
+            DirTable T;
             T.ngroups = (int)g.size();
             T.cmax = cmax;
             T.smem = sm_dir;
-            if (T.groups) {  // a rebuild (wcns_set_shape): the old table goes
-                c->owned.erase(std::remove(c->owned.begin(), c->owned.end(), (void *)T.groups), c->owned.end());
-                cudaFree(T.groups);
-            }
             T.groups = c->up(g);
-            size_t sm = sm_dir;
-            size_t &acc = pass == 0 ? inv_smem : pass == 1 ? vis_smem : pass == 2 ? inv_mx_smem : pass == 3 ? vis_mx_smem : adj_smem;
-            acc = std::max(acc, sm);
+            news.push_back({pass == 0 ? &L.inv[dir] : pass == 1 ? &L.vis[dir] : pass == 2 ? &L.inv_mx[dir] : pass == 3 ? &L.vis_mx[dir] : &L.adj[dir], T});
+            smem[pass] = std::max(smem[pass], sm_dir);
         }
     }
-    if (inv_smem > 227 * 1024 || vis_smem > 227 * 1024) { set_err("line too long for shared memory"); return WCNS_ERR_ARGUMENT; }
+    for (int pass = 0; pass < 4; pass++)
+        if (smem[pass] > 227 * 1024) { set_err("line too long for shared memory"); return give_up(WCNS_ERR_ARGUMENT); }
+    if (int rc = c->uploads_done()) return give_up(rc);
+    for (New &q : news) {
+        free_owned(c, q.old->groups);
+        *q.old = q.table;
+    }
     setup_rhs_invis_attrs(c->P.nflux);
     setup_rhs_vis_attrs();
-    if (inv_mx_smem > 227 * 1024 || vis_mx_smem > 227 * 1024) { set_err("line too long for shared memory"); return WCNS_ERR_ARGUMENT; }
     setup_rhs_mx_attrs();
     L.inv_cap = inv_cap;
     L.vis_cap = vis_cap;
@@ -883,6 +906,7 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
         L.hblocks = hbl;
     }
     rc = build_tables(c);
+    if (!rc) rc = c->uploads_done();
     if (rc) { delete c; return rc; }
     if (!L.sweep_plane && !L.wide)
         if (int rc2 = pm_alloc(c)) { delete c; return rc2; }
@@ -961,6 +985,7 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
         if (L.nwall) {
             L.walls = c->up(walls);
             L.wall_xyz = c->up(wxyz);
+            if (int rc2 = c->uploads_done()) { delete c; return rc2; }
             CK(cudaMalloc(&L.wall_pf, sizeof(double) * 3 * (size_t)npt));
             c->owned.push_back(L.wall_pf);
             CK(cudaMalloc(&L.wall_quad, sizeof(double) * 6 * (size_t)std::max(nq, 1LL)));
@@ -1676,9 +1701,9 @@ static int apply_shape(WcnsContext *c, const int *shape) {
             wide_free(c);
         }
     }
+    drop_graph(c);  // before the tables that it holds go
     if (shape[2] != L.inv_cap || shape[3] != L.vis_cap)
         if (int rc = build_line_tables(c, shape[2], shape[3])) return rc;
-    drop_graph(c);
     return 0;
 }
 
