@@ -47,6 +47,12 @@ class Hog:
             self.rt.cudaFree(p)
 
 
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
 def _check(g, ref):
     np.testing.assert_array_equal(g.step(2), ref.step(2))
     for nb in range(1, len(g.dims) + 1):
@@ -68,3 +74,44 @@ def test_line_tables_without_memory():
     _check(g, ref)
     g.set_shape(shape[:2] + [2, 2])  # with memory it is taken
     _check(g, ref)
+
+
+@pytest.mark.parametrize("form", ["clustered", "wide"])
+def test_autotune_without_memory_for_another_form(form):
+    """Room for the tuner's copy of dq, not for the other form's arrays (25 MB of the
+    clustered sweeps, 12 MB of the wide ones): the form in use stays, with the arrays
+    and the captured step that belong to it."""
+    from wcns_b200.solver import Wcns, WcnsError
+    case = perturbed(cases.vortex_case(ni=65, nj=24, nk=16))
+    g, ref = Wcns(case), Wcns(case)
+    if form == "clustered":
+        for h in (g, ref):
+            h.set_shape([8, 0] + h.shape[2:])
+    assert g.sweep_mode() == form
+    shape = g.shape
+    g.step(1), ref.step(1)
+    with Hog(leave=6 << 20):
+        if form == "clustered":
+            with pytest.raises(WcnsError):
+                g.autotune(1)
+            assert g.shape == shape
+        else:  # the lines per CTA are tuned all the same
+            g.autotune(1)
+        assert g.sweep_mode() == form
+    _check(g, ref)
+
+
+def test_autotune_keeps_only_the_arrays_of_the_form_it_takes():
+    from wcns_b200.solver import Wcns
+    case = perturbed(cases.vortex_case(ni=600, nj=48, nk=36))
+    g = Wcns(case)
+    assert g.sweep_mode() == "wide"
+    g.step(1)
+    before = _free()
+    g.set_shape([16, 0] + g.shape[2:])  # the clustered arrays are 745 MB, the wide ones 346
+    g.step(1)
+    assert before - _free() < 500 << 20
+    g.autotune(1)
+    assert before - _free() < (100 if g.sweep_mode() == "wide" else 500) << 20
+    g.set_shape([0, 0] + g.shape[2:])
+    assert before - _free() < 100 << 20

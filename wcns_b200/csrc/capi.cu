@@ -284,10 +284,7 @@ static void free_owned(WcnsContext *c, void *p) {
 // 0.55 against 2.25).
 constexpr int SWEEP_SMALL_PLANES = 35;
 
-// The wide cooperative sweeps' chunks and arrays (and the SA model's when it
-// is set up); L.wide points to them.  -1: the blocks cannot be swept wide;
-// a CUDA error code when an allocation fails.
-static int wide_alloc(WcnsContext *c) {
+static int wide_alloc_arrays(WcnsContext *c) {
     LaunchCtx &L = c->L;
     if (c->wide) {
         L.wide = c->wide.get();
@@ -319,11 +316,21 @@ static int wide_alloc(WcnsContext *c) {
     return 0;
 }
 
+// The wide cooperative sweeps' chunks and arrays (and the SA model's when it
+// is set up); L.wide points to them.  -1: the blocks cannot be swept wide;
+// a CUDA error code when an allocation fails, which leaves nothing behind.
+static int wide_alloc(WcnsContext *c) {
+    const size_t had = c->owned.size();
+    const int rc = wide_alloc_arrays(c);
+    if (rc > 0)
+        while (c->owned.size() > had) free_owned(c, c->owned.back());
+    return rc;
+}
+
 // The clustered sweeps' arrays, plane-major: dq (5 planes of values), the
 // static records (SR_N per cell) and three dynamic records (DYN_N per cell);
 // the memset leaves zero the records that no kernel ever writes.  A context
-// that sweeps wide has them from the first time that a cluster shape is asked
-// for.
+// that sweeps wide has them while it is tuned.
 static int pm_alloc(WcnsContext *c) {
     if (c->pm_pool) return 0;
     const size_t pmbytes = sizeof(double) * (size_t)(5 + SR_N + 3 * DYN_N) * (size_t)c->total_pm;
@@ -353,6 +360,11 @@ static int pm_layout(WcnsContext *c, int csize) {
     return 0;
 }
 
+static void pm_free(WcnsContext *c) {
+    if (c->pm_pool) cudaFree(c->pm_pool);
+    c->pm_pool = nullptr;
+}
+
 static void wide_free(WcnsContext *c) {
     if (!c->wide) return;
     WideSweep &W = *c->wide;
@@ -372,7 +384,10 @@ static void wide_free(WcnsContext *c) {
 // memory.  Longer lines than MAX_LINE are refused, as ever: nothing is tested there.
 constexpr int MAX_LINE = 997;
 
-static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
+// `passes`: bits of the tables to build, all of them unless a tuner tries one kernel.
+enum : int { PASS_ALL = 31 };
+
+static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap, int passes = PASS_ALL) {
     LaunchCtx &L = c->L;
     const int nbk = (int)c->blk.size();
     const bool sections = c->P.nscheme == 41 || c->P.nscheme == 42;
@@ -387,6 +402,7 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap) {
     };
     for (int dir = 0; dir < 3; dir++) {
         for (int pass = 0; pass < 5; pass++) {  // 0 inviscid, 1 viscous, 2 and 3 the same in mixed precision, 4 the adjoint's operators
+            if (!(passes >> pass & 1)) continue;
             std::vector<LineGroup> g;
             size_t sm_dir = 0;
             int cmax = 0;
@@ -728,12 +744,8 @@ static int build_tables(WcnsContext *c) {
         for (int b = 0; b < nbk; b++) planes = std::max(planes, c->blk[b].d.ni + c->blk[b].d.nj + c->blk[b].d.nk - 2);
         const bool prefer_wide = !clustered || (planes > SWEEP_SMALL_PLANES && !getenv("WCNS_SWEEP_CLUSTER"));
         if (prefer_wide && !want_plane) {
-            const size_t had = c->owned.size();
-            if (int rc = wide_alloc(c); rc > 0) {
-                while (c->owned.size() > had) free_owned(c, c->owned.back());
-                if (!clustered) return rc;  // no memory, and no other form
-                cudaGetLastError();
-            }
+            const int rc = wide_alloc(c);
+            if (rc > 0 && !clustered) return rc;  // no memory, and no other form
         }
         L.sweep_plane = !clustered && !L.wide ? 1 : 0;
     }
@@ -1689,6 +1701,8 @@ static int apply_shape(WcnsContext *c, const int *shape) {
                     if (rc < 0) set_err("wcns_set_shape: the blocks cannot be swept wide");
                     return rc < 0 ? WCNS_ERR_ARGUMENT : rc;
                 }
+                drop_graph(c);
+                pm_free(c);
             }
         } else if (L.wide || shape[0] != L.sweep_cluster || shape[1] != L.sweep_fine) {
             if (setup_sweep_exact(L, shape[0], shape[1])) {
@@ -1698,6 +1712,7 @@ static int apply_shape(WcnsContext *c, const int *shape) {
             }
             if (int rc = pm_alloc(c)) return rc;
             if (int rc = pm_layout(c, L.sweep_cluster)) return rc;
+            drop_graph(c);
             wide_free(c);
         }
     }
@@ -1750,6 +1765,48 @@ static double time_reps(WcnsContext *c, int reps, const double *saved, Body body
     return total / reps;
 }
 
+// The sweep forms of wcns_autotune: every cluster shape, and the wide sweeps.  Leaves
+// the fastest in use, its shape in best[0..1]; on an error the form it began with.
+static int tune_sweeps(WcnsContext *c, int reps, const double *saved, int *best, double *best_ms) {
+    LaunchCtx &L = c->L;
+    const int first[2] = {best[0], best[1]};  // first[0] == 0: wide
+    double tbest = 1e300;
+    const int cls[5] = {1, 2, 4, 8, 16};
+    int rc = 0;
+    L.wide = nullptr;
+    for (int fine = 1; fine >= 0; fine--)
+        for (int q = 0; q < 5; q++) {
+            if (rc || setup_sweep_exact(L, cls[q], fine)) continue;
+            rc = pm_layout(c, L.sweep_cluster);
+            if (rc) continue;
+            const double t = time_reps(c, reps, saved, [&] { launch_lhs(L); });
+            if (t < tbest) { tbest = t; best[0] = cls[q]; best[1] = fine; }
+        }
+    L.wide = c->wide.get();
+    if (!rc) {
+        const int wr = wide_alloc(c);
+        if (wr > 0) rc = wr;
+        if (wr == 0) {
+            const double t = time_reps(c, reps, saved, [&] { launch_lhs(L); });
+            if (t < tbest) { tbest = t; best[0] = 0; best[1] = 0; }
+        }
+    }
+    if (rc) {
+        best[0] = first[0];
+        best[1] = first[1];
+    }
+    // the arrays of the form that is not taken go
+    if (best[0] > 0) {
+        setup_sweep_exact(L, best[0], best[1]);
+        if (const int lr = pm_layout(c, L.sweep_cluster)) rc = rc ? rc : lr;
+        wide_free(c);
+    } else {
+        pm_free(c);
+    }
+    *best_ms = tbest;
+    return rc;
+}
+
 // Times every candidate shape on the context's current state with the
 // phases it shapes (the LU-SGS phase for the sweep shape, the inviscid and
 // viscous residual for the line caps), keeps the fastest, and returns it in
@@ -1759,60 +1816,39 @@ extern "C" int wcns_autotune(WcnsContext *c, int reps, int *shape, double *ms) {
     if (!c || !shape || reps < 1) { set_err("wcns_autotune: invalid argument"); return WCNS_ERR_ARGUMENT; }
     LaunchCtx &L = c->L;
     CK(cudaStreamSynchronize(c->stream));
-    double *saved = nullptr;
     const size_t bytes = sizeof(double) * 5 * (size_t)c->total;
-    CK(cudaMalloc(&saved, bytes));
-    CK(cudaMemcpy(saved, c->F.f[F_DQ1], bytes, cudaMemcpyDeviceToDevice));
+    struct Copy {
+        double *p = nullptr;
+        ~Copy() { if (p) cudaFree(p); }
+    } copy;
+    CK(cudaMalloc(&copy.p, bytes));
+    const double *saved = copy.p;
+    CK(cudaMemcpy(copy.p, c->F.f[F_DQ1], bytes, cudaMemcpyDeviceToDevice));
+    drop_graph(c);
     int best[4];
     wcns_get_shape(c, best);
     double best_ms[3] = {0.0, 0.0, 0.0};
-    // the LU-SGS sweep form and shape: every cluster shape, and the wide sweeps
-    if (can_cluster(c) && !L.sweep_plane && pm_alloc(c) == 0) {
-        double tbest = 1e300;
-        const bool was_wide = L.wide != nullptr;
-        L.wide = nullptr;
-        const int cls[5] = {1, 2, 4, 8, 16};
-        for (int fine = 1; fine >= 0; fine--)
-            for (int q = 0; q < 5; q++) {
-                int cand[4] = {cls[q], fine, best[2], best[3]};
-                if (setup_sweep_exact(L, cand[0], cand[1])) continue;
-                if (int rc = pm_layout(c, L.sweep_cluster)) { cudaFree(saved); return rc; }
-                const double t = time_reps(c, reps, saved, [&] { launch_lhs(L); });
-                if (t < tbest) { tbest = t; best[0] = cand[0]; best[1] = cand[1]; }
-            }
-        if (was_wide) L.wide = c->wide.get();
-        const int wr = wide_alloc(c);
-        if (wr > 0) { cudaFree(saved); return wr; }
-        if (wr == 0) {
-            const double t = time_reps(c, reps, saved, [&] { launch_lhs(L); });
-            if (t < tbest) { tbest = t; best[0] = 0; best[1] = 0; }
-        }
-        if (best[0] > 0) {
-            setup_sweep_exact(L, best[0], best[1]);
-            if (int rc = pm_layout(c, L.sweep_cluster)) return rc;
-            wide_free(c);
-        }
-        best_ms[0] = tbest;
-    }
-    // lines per CTA of the residual kernels
+    int rc = 0;
+    if (can_cluster(c) && !L.sweep_plane && pm_alloc(c) == 0) rc = tune_sweeps(c, reps, saved, best, &best_ms[0]);
+    // lines per CTA of the residual kernels: a candidate needs the tables of the
+    // kernel it is timed on, the last call builds them all
     const int caps[4] = {4, 8, 16, 32};
-    for (int vis = 0; vis <= (c->P.nvis == 1 ? 1 : 0); vis++) {
+    for (int vis = 0; vis <= (c->P.nvis == 1 ? 1 : 0) && !rc; vis++) {
         if (vis) launch_node_derivatives(L);
         double tbest = 1e300;
         int kbest = vis ? best[3] : best[2];
         for (int q = 0; q < 4; q++) {
             const int ic = vis ? best[2] : caps[q], vc = vis ? caps[q] : best[3];
-            if (build_line_tables(c, ic, vc)) continue;
+            if (build_line_tables(c, ic, vc, 1 << (vis + (L.mixed ? 2 : 0)))) continue;
             const double t = time_reps(c, reps, saved, [&] { launch_rhs_dirs(L, vis == 1); });
             if (t < tbest) { tbest = t; kbest = caps[q]; }
         }
         best[vis ? 3 : 2] = kbest;
         best_ms[vis ? 2 : 1] = tbest;
-        build_line_tables(c, best[2], best[3]);
     }
+    if (!rc) rc = build_line_tables(c, best[2], best[3]);
     cudaMemcpy(c->F.f[F_DQ1], saved, bytes, cudaMemcpyDeviceToDevice);
-    cudaFree(saved);
-    drop_graph(c);
+    if (rc) return rc;
     CK(cudaGetLastError());
     for (int q = 0; q < 4; q++) shape[q] = best[q];
     if (ms)
