@@ -162,3 +162,21 @@ def test_cluster_size_changed_between_steps():
     for other in out[1:]:
         for x, y in zip(out[0], other):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shapes", [((16, 1), (4, 0), (8, 1)), ((2, 0), (16, 1), (4, 0))], ids=str)
+def test_every_cluster_size_in_turn_equals_the_wide_sweeps(shapes):
+    """Each step runs the cluster size it is meant to run (no refusal is passed over),
+    and the slots of one size leave nothing for the next."""
+    from tests.helpers import perturbed
+    from wcns_b200.solver import Wcns
+    case = perturbed(cases.vortex_case(ni=30, nj=18, nk=11, nscheme=4, nflux=1))
+    ref, g = Wcns(case), Wcns(case)
+    assert ref.sweep_mode() == "wide"
+    for s in shapes:
+        g.set_shape(list(s) + g.shape[2:])
+        assert g.sweep_mode() == "clustered" and tuple(g.shape[:2]) == s
+        np.testing.assert_array_equal(g.step(1), ref.step(1))
+    for f in ("r", "u", "v", "w", "p"):
+        np.testing.assert_array_equal(g.get(f, 1), ref.get(f, 1))
