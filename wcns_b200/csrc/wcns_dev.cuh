@@ -296,17 +296,19 @@ __device__ __forceinline__ int flux_vl_pn(const DevParams &P, const double *prim
 
 // a / b from r = 1 / b: the quotient of the two rounded values corrected by
 // its remainder (Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990), the rounded quotient but for cases rarer than
-// one in 1e12.  For b and 1 / b finite and normal; a division costs a dozen
-// instructions and a branch, this three.
+// System/6000 processor", 1990): the rounded quotient for every sample of
+// tests/test_device_arithmetic.py.  For b and 1 / b finite and normal, and a far from
+// the subnormal numbers; an infinite a gives NaN, not an infinity, and -0 gives +0.  A
+// division costs a dozen instructions and a branch, this three.
 __device__ __forceinline__ double div_by(double a, double b, double r) {
     const double q = a * r;
     return fma(fma(-q, b, a), r, q);
 }
 
 // 1 / b and 1 / sqrt(x) of normal numbers from the hardware's approximation
-// (relative error below 2^-20) by one step of the iteration of third order
-// (Householder), to within an ulp or two: where the last bit does not matter.
+// (relative error below 2^-19.9) by one step of the iteration of third order
+// (Householder), to 0.51 and 1.02 ulp: where the last bit does not matter.  Zero, an
+// infinity or a subnormal number gives NaN or an infinity, where 1 / b may give zero.
 __device__ __forceinline__ double recip(double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
