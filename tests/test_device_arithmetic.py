@@ -119,11 +119,13 @@ def test_div_by(probe, b):
 
 def test_special_values(probe):
     """What the comments state: NaN stays NaN, a negative root is NaN, and where an
-    operand is zero, infinite or subnormal the short forms give no finite number."""
+    operand is zero, infinite or subnormal recip and recip_sqrt give no finite number;
+    div_by gives what a division gives."""
     inf, nan = np.inf, np.nan
     assert np.isnan(probe(RECIP, [0.0, -0.0, inf, -inf, nan])).all()
     assert np.isnan(probe(RSQRT, [0.0, -0.0, inf, nan, -1.0, -inf])).all()
     assert not np.isfinite(probe(RECIP, [1e-310, -1e-310])).any()
     assert not np.isfinite(probe(RSQRT, [1e-310])).any()
-    assert np.isnan(probe(DIV, [inf, -inf, nan], 1920.0)).all()
-    assert (probe(DIV, [0.0, -0.0], 24.0) == 0.0).all()
+    a = np.repeat([inf, -inf, nan, 0.0, -0.0, 1.5, -1.5], 6)
+    b = np.tile([1920.0, -24.0, 0.0, inf, -inf, nan], 7)
+    np.testing.assert_array_equal(probe(DIV, a, b), probe(CUDA_DIV, a, b))

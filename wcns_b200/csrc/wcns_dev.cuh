@@ -297,12 +297,15 @@ __device__ __forceinline__ int flux_vl_pn(const DevParams &P, const double *prim
 // a / b from r = 1 / b: the quotient of the two rounded values corrected by
 // its remainder (Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990): the rounded quotient for every sample of
-// tests/test_device_arithmetic.py.  For b and 1 / b finite and normal, and a far from
-// the subnormal numbers; an infinite a gives NaN, not an infinity, and -0 gives +0.  A
-// division costs a dozen instructions and a branch, this three.
+// tests/test_device_arithmetic.py.  For b and 1 / b normal and a far from the subnormal
+// numbers; where a, b or r is zero or infinite the correction is NaN and the first
+// quotient is what a division gives (-0 / b gives +0).  A division costs a dozen
+// instructions and a branch, this six; without the last step the residual phases take
+// 1.3 % less (channel: viscous 1345 for 1364 us, inviscid 1136 for 1148) and turn an
+// infinite derivative into an undefined one.
 __device__ __forceinline__ double div_by(double a, double b, double r) {
-    const double q = a * r;
-    return fma(fma(-q, b, a), r, q);
+    const double q = a * r, c = fma(fma(-q, b, a), r, q);
+    return c == c ? c : q;
 }
 
 // 1 / b and 1 / sqrt(x) of normal numbers from the hardware's approximation
