@@ -62,3 +62,9 @@ def _compare(field, values, points, nscheme, nflux, nvis):
 def test_viscous(field):
     _compare(field, (INF, -INF, float("nan"), 1e60), POINTS, 4, 1, 1)
 
+
+@pytest.mark.parametrize("nflux", [1, 2, 3])
+@pytest.mark.parametrize("nscheme", [4, 41, 42])
+@pytest.mark.parametrize("field", ["r", "u", "p"])
+def test_inviscid(field, nscheme, nflux):
+    _compare(field, (INF, float("nan"), 1e30, 1e60), POINTS, nscheme, nflux, 0)

@@ -46,7 +46,13 @@
 // The central part of the fluxes and the differences keep the reference's
 // operations and their order: where the flow is uniform they cancel to
 // round-off, which is compared.  The weights, and in the Roe flux all that is
-// multiplied by the jump, are free of that.
+// multiplied by the jump, are free of that.  Where a sum of weights, a sound speed or a
+// Roe flux leaves the range of the short forms, the CTA ends its march and does the rest
+// of its lines with the reference's divisions (inv_rest), so that special values reach
+// the residual as they do in the reference.  The checks take 0.5 % (channel 1148 to
+// 1154 us); a branch to the divisions in the loop took 6 % there and 9 % on 64 small
+// blocks, a call for the chunk 17 %, by the registers they hold.  A state that is
+// undefined everywhere takes 1.5 ms where the channel of 0.5 M points takes 0.24.
 #include <algorithm>
 
 #include "wcns_dev.cuh"
@@ -84,9 +90,12 @@ struct InvLine {  // one line's view of the ring
 };
 
 // The state at a half node from the five points around `c0` (WCNSE5.f90:2-206):
-// left states from point h, right states from point h+1.
+// left states from point h, right states from point h+1.  top: the largest sum of
+// weights so far (its high word; NaN above all numbers).  From TOP_WEIGHT, 1e300, on
+// the products and the reciprocal may leave the range.
+constexpr unsigned TOP_WEIGHT = 0x7e37e43cu;
 template <bool LEFT>
-__device__ __forceinline__ double wcns_state(double m2, double m1, double c0, double p1, double p2) {
+__device__ __forceinline__ double wcns_state(double m2, double m1, double c0, double p1, double p2, unsigned &top) {
     const double EPS = 1.0e-6;
     const double g0 = 0.5 * (m2 - 4.0 * m1 + 3.0 * c0), g1 = 0.5 * (p1 - m1), g2 = 0.5 * (-3.0 * c0 + 4.0 * p1 - p2);
     const double s0 = m2 - 2.0 * m1 + c0, s1 = m1 - 2.0 * c0 + p1, s2 = c0 - 2.0 * p1 + p2;
@@ -96,7 +105,30 @@ __device__ __forceinline__ double wcns_state(double m2, double m1, double c0, do
     const double a0 = fma(four, g0, s0), a1 = fma(four, g1, s1), a2 = fma(four, g2, s2);
     // weights 1/16, 10/16, 5/16 (left), 5/16, 10/16, 1/16 (right)
     const double w0 = LEFT ? e1 * e2 : 5.0 * (e1 * e2), w1 = 10.0 * (e0 * e2), w2 = LEFT ? 5.0 * (e0 * e1) : e0 * e1;
-    return c0 + 0.125 * (fma(w2, a2, fma(w1, a1, w0 * a0)) * recip(w0 + w1 + w2));
+    const double sum = w0 + w1 + w2;
+    top = max(top, (unsigned)__double2hiint(sum));
+    return c0 + 0.125 * (fma(w2, a2, fma(w1, a1, w0 * a0)) * recip(sum));
+}
+// The same with the reference's divisions, which overflow at far larger values and
+// pass infinities on.
+template <bool LEFT>
+__device__ __forceinline__ double wcns_state_div(double m2, double m1, double c0, double p1, double p2) {
+    const double g[3] = {0.5 * (m2 - 4.0 * m1 + 3.0 * c0), 0.5 * (p1 - m1), 0.5 * (-3.0 * c0 + 4.0 * p1 - p2)};
+    const double s[3] = {m2 - 2.0 * m1 + c0, m1 - 2.0 * c0 + p1, c0 - 2.0 * p1 + p2};
+    const double cl[3] = {1.0 / 16.0, 10.0 / 16.0, 5.0 / 16.0}, four = LEFT ? 4.0 : -4.0;
+    double b[3], a = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double t = 1.0e-6 + (g[k] * g[k] + s[k] * s[k]);
+        b[k] = cl[LEFT ? k : 2 - k] / (t * t);
+    }
+    const double sum = b[0] + b[1] + b[2];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double x = b[k] / sum * (s[k] + four * g[k]);
+        a = k ? a + x : x;
+    }
+    return c0 + 0.125 * a;
 }
 
 // Boundary-section states (left WCNSE5.f90:2284-2459, right 2524-2705, which
@@ -104,10 +136,12 @@ __device__ __forceinline__ double wcns_state(double m2, double m1, double c0, do
 // points 1..4 (or n..n-3), the divisor and its reciprocal.  nscheme=42 has
 // second-order states at the first four half nodes (2967-2986, 3207-3226).
 enum : int { SEC_S1 = 0, SEC_S1_42 = 4, SEC_S2 = 8, SEC_S2R2 = 13, SEC_S3L2 = 14, SEC_C = 15, SEC_ROWS = 18, SEC_W = 6 };
+// A coefficient 0.0 stands for a point that the reference's formula has not, -0.0 for
+// its explicit product with zero.
 #define SEC_ROW(a, b, c, d, den) a, b, c, d, den, 1.0 / (den)
 __constant__ double sec_table[SEC_ROWS * SEC_W] = {
     // s1 at half nodes 0..3, nscheme 41
-    SEC_ROW(3.0, -1.0, 0.0, 0.0, 2.0), SEC_ROW(19.0, 25.0, -2.0, 0.0, 42.0), SEC_ROW(4.0, 3.0, 9.0, 2.0, 18.0), SEC_ROW(-2.0, 3.0, 3.0, 2.0, 6.0),
+    SEC_ROW(3.0, -1.0, -0.0, 0.0, 2.0), SEC_ROW(19.0, 25.0, -2.0, 0.0, 42.0), SEC_ROW(4.0, 3.0, 9.0, 2.0, 18.0), SEC_ROW(-2.0, 3.0, 3.0, 2.0, 6.0),
     // the same, nscheme 42
     SEC_ROW(677.0, -421.0, 99.0, 13.0, 368.0), SEC_ROW(5.0, 15.0, -5.0, 1.0, 16.0), SEC_ROW(-1.0, 9.0, 9.0, -1.0, 16.0), SEC_ROW(1.0, -5.0, 15.0, 5.0, 16.0),
     // s2 at half nodes 1..5 (left states at the left end, right ones at the right end)
@@ -139,13 +173,164 @@ __device__ __forceinline__ int closure_right(const InvLine &L, int h, bool &end)
     return L.ied < L.n && h >= L.n - 2 ? SEC_C + L.n - h : -1;
 }
 
+// Where an item's two states come from: a row of the table and the end it counts from
+// or, -1, the interior scheme and its closures.  Item: a half node (sec < 0), or a flux
+// of the ends' sections.  Sections 0..25: at the left end s1 at half nodes 0..3, s2 at
+// 1..5, s3 at 1..4; at the right end s4, s5, s6 likewise, counting down from n.
+struct InvItem {
+    int h, isec, rowl, rowr;
+    bool endl, endr;
+    // false: the line has no section there
+    __device__ __forceinline__ bool set(int nscheme, const InvLine &L, int half, int sec) {
+        h = half;
+        isec = sec;
+        rowl = rowr = -1;
+        endl = endr = false;
+        if (sec < 0) return true;
+        const bool right = sec >= 13;
+        if (right ? L.ied >= L.n : L.ist <= 1) return false;
+        const int q = right ? sec - 13 : sec, s1 = nscheme == 42 ? SEC_S1_42 : SEC_S1;
+        int o;  // half nodes from the end
+        if (q < 4) {
+            o = q;
+            rowl = rowr = s1 + o;
+        } else if (q < 9) {
+            o = q - 3;
+            rowl = SEC_S2 + o - 1;
+            rowr = o == 2 ? SEC_S2R2 : rowl;
+        } else {
+            o = q - 8;
+            rowl = o == 2 ? SEC_S3L2 : SEC_S2 + o - 1;
+        }
+        h = o;
+        if (right) {
+            h = L.n - o;
+            const int x = rowl;
+            rowl = rowr;
+            rowr = x;
+            endl = endr = true;
+            // s6: the left state as the left sections left it where they
+            // ran (h <= 5), otherwise the interior scheme's
+            if (q >= 9 && L.ist > 1 && h <= 5) {
+                endl = false;
+                rowl = h == 0 ? s1 : h == 2 ? SEC_S3L2 : SEC_S2 + h - 1;
+            }
+        }
+        return true;
+    }
+};
+
 __device__ __forceinline__ void inv_copy8(double *dst, const double *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
+// The difference at the o-th point from a flagged end, of one component of the line's
+// section fluxes.  s1, s4 hold f(k) and s2, s3, s5, s6 f(k + 1), k half nodes from the end.
+__device__ __forceinline__ double section_difference(const double *s, bool right, int o) {
+    if (right) s += 13 * 5;
+    const double *a = s, *b = s + 4 * 5, *c = s + 9 * 5;
+    const double d = o == 0 ? -23.0 * a[0] + 21.0 * a[5] + 3.0 * a[10] - 1.0 * a[15]
+                   : o == 1 ? -22.0 * b[0] + 17.0 * b[5] + 9.0 * b[10] - 5.0 * b[15] + b[20] : c[0] - 27.0 * c[5] + 27.0 * c[10] - c[15];
+    return (right ? -d : d) / 24.0;
+}
+
+// The points done+1..n of a group's lines with the reference's divisions, from memory: C
+// points at a time, their half nodes' fluxes in `fr` (C + 5 per line), the sections'
+// in `secf`.  Called by all threads of the CTA when nothing of the march is needed any
+// more, so that it costs the march no registers.  Returns the thread's c^2 failures at
+// the half nodes from h0 on (and the sections after it), each counted once.
+template <int dir, int NFLUX>
+__device__ __noinline__ int inv_rest(const DevParams *P, const DevFields *F, const DevBlock *B, const LineGroup *G, int done, int h0, int C, double *fr,
+                                     double *secf, const double *sec) {
+    const int n = dimof(*B, dir), NL = G->nl, st = (int)dstride(*B, dir);
+    constexpr int a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
+    const int lstep = (int)dstride(*B, a1);
+    int o3[3];
+    o3[a1] = G->a0;
+    o3[a2] = G->b;
+    o3[dir] = 0;
+    const int base = (int)gidx(*B, o3[0], o3[1], o3[2]);
+    const bool scheme4x = P->nscheme == 41 || P->nscheme == 42;
+    int bad = 0, hc = h0;  // half nodes below hc have been counted
+    auto line = [&](int ln) {
+        InvLine L;
+        L.n = n;
+        const double *rho = F->f[F_R] + base + ln * lstep;
+        L.ist = rho[-2 * st] < SMALL ? 2 : 0;
+        L.ied = rho[(n + 3) * st] < SMALL ? n - 2 : n;
+        return L;
+    };
+    // one item's flux
+    auto item = [&](int ln, int half, int isec, double *f) {
+        const InvLine L = line(ln);
+        InvItem I;
+        if (!I.set(P->nscheme, L, half, isec)) return;
+        const int h = I.h, g = base + ln * lstep;
+        auto q = [&](int m, int p) { return F->f[F_R + m][g + p * st]; };
+        if (I.rowl < 0) I.rowl = closure_left(L, h, I.endl);
+        if (I.rowr < 0) I.rowr = closure_right(L, h, I.endr);
+        auto row = [&](int rw, int m, bool right) {  // a row's state, of the points that its formula has
+            const double *c = sec + rw * SEC_W;
+            double a = -0.0;
+            for (int k = 0; k < 4; k++)
+                if (__double_as_longlong(c[k]) != 0) a = a + c[k] * q(m, right ? n - k : 1 + k);
+            return a / c[4];
+        };
+        double ql[5], qr[5], fl[5];
+#pragma unroll
+        for (int m = 0; m < 5; m++) {
+            ql[m] = I.rowl >= 0 ? row(I.rowl, m, I.endl) : wcns_state_div<true>(q(m, h - 2), q(m, h - 1), q(m, h), q(m, h + 1), q(m, h + 2));
+            qr[m] = I.rowr >= 0 ? row(I.rowr, m, I.endr) : wcns_state_div<false>(q(m, h - 1), q(m, h), q(m, h + 1), q(m, h + 2), q(m, h + 3));
+        }
+        const bool badl = ql[0] <= RMIN_LIMIT || ql[4] <= PMIN_LIMIT, badr = qr[0] <= RMIN_LIMIT || qr[4] <= PMIN_LIMIT;
+        const bool same = isec >= 0 && I.rowl == I.rowr && I.rowl < SEC_S2;
+        const int ia = h > 1 ? h : 1, ib = h + 1 < n ? h + 1 : n;
+        const int la = same && I.endl ? 1 : ia, lb = same ? (I.endl ? h : h + 1) : ia, ra = same ? la : ib, rb = same ? lb : ib;
+#pragma unroll
+        for (int m = 0; m < 5; m++) {
+            if (badl) ql[m] = (q(m, la) + q(m, lb)) / 2.0;
+            if (badr) qr[m] = (q(m, ra) + q(m, rb)) / 2.0;
+        }
+        double k[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            auto a = [&](int p) { return F->f[F_KCX + 3 * dir + d][g + p * st]; };
+            k[d] = value_half_node_at(a, n, h);
+        }
+        const int b = NFLUX == 3 ? flux_roe_div(P->gama, P->efix, k[0], k[1], k[2], ql, qr, fl)
+                                 : flux_split<NFLUX>(*P, ql, qr, k[0], k[1], k[2], 0.0, fl);
+        if (isec < 0 ? h >= hc : isec >= 13 || h0 == 0) bad += b;
+#pragma unroll
+        for (int m = 0; m < 5; m++) f[m] = fl[m];
+    };
+    __syncthreads();
+    if (scheme4x)
+        for (int e = threadIdx.x; e < 26 * NL; e += INV_THREADS) item(e % NL, 0, e / NL, secf + (e % NL * 26 + e / NL) * 5);
+    for (int l0 = done + 1; l0 <= n; l0 += C) {
+        const int l1 = l0 + C - 1 < n ? l0 + C - 1 : n;
+        // the half nodes of these points' differences: l-3..l+2, 0..4 and n-4..n at the ends
+        const int ha = max(0, min(l0 - 3, n - 4)), hb = min(n, max(l1 + 2, 4));
+        __syncthreads();
+        for (int e = threadIdx.x; e < (hb - ha + 1) * NL; e += INV_THREADS) item(e % NL, ha + e / NL, -1, fr + e * 5);
+        hc = max(hc, hb + 1);
+        __syncthreads();
+        for (int e = threadIdx.x; e < (l1 - l0 + 1) * NL; e += INV_THREADS) {
+            const int ln = e % NL, l = l0 + e / NL, gi = base + ln * lstep + l * st;
+            const InvLine L = line(ln);
+            const int end = !scheme4x ? 0 : L.ied < n && l >= n - 2 ? 2 : L.ist > 1 && l <= 3 ? 1 : 0;
+            for (int m = 0; m < 5; m++) {
+                auto fa = [&](int hh) { return fr[((hh - ha) * NL + ln) * 5 + m]; };
+                const double v = end ? section_difference(secf + ln * 130 + m, end == 2, end == 2 ? n - l : l - 1) : flux_dxyz_at(fa, n, l);
+                F->f[F_DQ1 + m][gi] = F->f[F_DQ1 + m][gi] + v;
+            }
+        }
+    }
+    return bad;
+}
+
 // dq += dF in place.
 template <int dir, int NFLUX>
-__global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(DevParams P, DevFields F, const DevBlock *__restrict__ blocks,
+__global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(const __grid_constant__ DevParams P, const __grid_constant__ DevFields F, const DevBlock *__restrict__ blocks,
                                                        const LineGroup *__restrict__ groups, int cmax, int *err) {
     extern __shared__ __align__(16) double smem[];
     const LineGroup G = groups[blockIdx.x];
@@ -204,6 +389,7 @@ __global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(DevParams P
     anyr = __syncthreads_or(scheme4x && anyr);
     const double gama1 = P.gama - 1.0, gama1_1 = 1.0 / gama1;
     int nbad = 0;
+    bool rest = false;
     InvLine L;
     L.ring = smem + ln * INV_PITCH;
     L.RP = RP;
@@ -229,67 +415,37 @@ __global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(DevParams P
         // line-fastest, the lanes of a warp take the same position on neighbouring
         // lines and follow one control path
         const int nl13 = h0 == 0 && anyl ? 13 : 0, T = len + nl13 + (last && anyr ? 13 : 0);
+        bool odd = false;  // an item left the range of the short forms
+        int bad = 0;
         for (int t = c; t < T && c < TC; t += TC) {
             double ql[5], qr[5], fl[5];
-            // Where the two states come from: a row of the table (and the end it
-            // counts from) or, -1, the interior scheme.  Sections 0..25: at the
-            // left end s1 at half nodes 0..3, s2 at 1..5, s3 at 1..4; at the right
-            // end s4, s5, s6 likewise, counting down from n.
-            int h = h0 + t, rowl = -1, rowr = -1, isec = -1;
-            bool endl = false, endr = false;
-            if (t >= len) {
-                int sidx = t - len + (nl13 ? 0 : 13);
-                const bool right = sidx >= 13;
-                isec = sidx;
-                if (right ? L.ied >= n : L.ist <= 1) continue;
-                if (right) sidx -= 13;
-                const int s1 = P.nscheme == 42 ? SEC_S1_42 : SEC_S1;
-                int o;  // half nodes from the end
-                if (sidx < 4) {
-                    o = sidx;
-                    rowl = rowr = s1 + o;
-                } else if (sidx < 9) {
-                    o = sidx - 3;
-                    rowl = SEC_S2 + o - 1;
-                    rowr = o == 2 ? SEC_S2R2 : rowl;
-                } else {
-                    o = sidx - 8;
-                    rowl = o == 2 ? SEC_S3L2 : SEC_S2 + o - 1;
-                }
-                h = o;
-                if (right) {
-                    h = n - o;
-                    const int x = rowl;
-                    rowl = rowr;
-                    rowr = x;
-                    endl = endr = true;
-                    // s6: the left state as the left sections left it where they
-                    // ran (h <= 5), otherwise the interior scheme's
-                    if (sidx >= 9 && L.ist > 1 && h <= 5) {
-                        endl = false;
-                        rowl = h == 0 ? s1 : h == 2 ? SEC_S3L2 : SEC_S2 + h - 1;
-                    }
-                }
-            }
+            InvItem I;
+            if (!I.set(P.nscheme, L, h0 + t, t < len ? -1 : t - len + (nl13 ? 0 : 13))) continue;
+            const int h = I.h, isec = I.isec;
+            int rowl = I.rowl, rowr = I.rowr;
+            bool endl = I.endl, endr = I.endr;
             if (rowl < 0) rowl = closure_left(L, h, endl);
             if (rowr < 0) rowr = closure_right(L, h, endr);
             const double *x0 = L.at(h - 2), *x1 = L.at(h - 1), *x2 = L.at(h), *x3 = L.at(h + 1), *x4 = L.at(h + 2), *x5 = L.at(h + 3);
+            unsigned top = 0;
             if (rowl < 0 && rowr < 0) {
 #pragma unroll
                 for (int m = 0; m < 5; m++) {
-                    ql[m] = wcns_state<true>(x0[m], x1[m], x2[m], x3[m], x4[m]);
-                    qr[m] = wcns_state<false>(x1[m], x2[m], x3[m], x4[m], x5[m]);
+                    ql[m] = wcns_state<true>(x0[m], x1[m], x2[m], x3[m], x4[m], top);
+                    qr[m] = wcns_state<false>(x1[m], x2[m], x3[m], x4[m], x5[m], top);
                 }
             } else {  // few items: one copy of the code for all variables
                 double tl[5], tr[5];
 #pragma unroll 1
                 for (int m = 0; m < 5; m++) {
-                    tl[m] = rowl < 0 ? wcns_state<true>(x0[m], x1[m], x2[m], x3[m], x4[m]) : sec_state(sec + rowl * SEC_W, L, m, endl);
-                    tr[m] = rowr < 0 ? wcns_state<false>(x1[m], x2[m], x3[m], x4[m], x5[m]) : sec_state(sec + rowr * SEC_W, L, m, endr);
+                    tl[m] = rowl < 0 ? wcns_state<true>(x0[m], x1[m], x2[m], x3[m], x4[m], top) : sec_state(sec + rowl * SEC_W, L, m, endl);
+                    tr[m] = rowr < 0 ? wcns_state<false>(x1[m], x2[m], x3[m], x4[m], x5[m], top) : sec_state(sec + rowr * SEC_W, L, m, endr);
+                    top = max(top, max((unsigned)__double2hiint(tl[m]) & 0x7fffffffu, (unsigned)__double2hiint(tr[m]) & 0x7fffffffu));
                 }
 #pragma unroll
                 for (int m = 0; m < 5; m++) { ql[m] = tl[m]; qr[m] = tr[m]; }
             }
+            odd = odd || top >= TOP_WEIGHT;
             // positivity fallback: the neighbouring point; in s1 and s4 means
             const bool badl = ql[0] <= RMIN_LIMIT || ql[4] <= PMIN_LIMIT, badr = qr[0] <= RMIN_LIMIT || qr[4] <= PMIN_LIMIT;
             const bool same = isec >= 0 && rowl == rowr && rowl < SEC_S2;
@@ -320,13 +476,17 @@ __global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(DevParams P
                 kz = (ca * ka[7] + cb * kb[7] + cc * kc[7] + cd * kd[7]) / 16.0;
             }
             const double kt = 0.0;  // kct=0, so every half-node value of kt is +0
-            if (NFLUX == 3) nbad += flux_roe(P, gama1_1, ql, qr, kx, ky, kz, kt, same, fl);
-            else nbad += flux_split<NFLUX>(P, ql, qr, kx, ky, kz, kt, fl);
+            if (NFLUX == 3) odd = !flux_roe(P, gama1_1, ql, qr, kx, ky, kz, kt, same, fl) || odd;
+            else bad += flux_split<NFLUX>(P, ql, qr, kx, ky, kz, kt, fl);
             double *f_ = isec < 0 ? fr + (wrap(fs + h - h0, FR) * NLP + ln) * INV_FP : secf + (ln * 26 + isec) * 5;
 #pragma unroll
             for (int m = 0; m < 5; m++) f_[m] = fl[m];
         }
-        __syncthreads();
+        if (__syncthreads_or(odd)) {
+            rest = true;
+            break;
+        }
+        nbad += bad;
         if (have < n + 3) {  // the next chunk's points, in place of the oldest
             int hi = h0 + len + C + 2;
             if (hi > n + 3) hi = n + 3;
@@ -360,17 +520,8 @@ __global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(DevParams P
 #pragma unroll 1
                 for (int m = 0; m < 5; m++) {
                     double v;
-                    if (right) {
-                        const double *s4 = sc + 13 * 5 + m, *s5 = sc + 17 * 5 + m, *s6 = sc + 22 * 5 + m;
-                        // section fluxes f(ni-h): s4[k] holds f(k), s5[k] and s6[k] hold f(k+1)
-                        if (l == n) v = -(-23.0 * s4[0] + 21.0 * s4[5] + 3.0 * s4[10] - 1.0 * s4[15]) / 24.0;
-                        else if (l == n - 1) v = -(-22.0 * s5[0] + 17.0 * s5[5] + 9.0 * s5[10] - 5.0 * s5[15] + s5[20]) / 24.0;
-                        else v = -(s6[0] - 27.0 * s6[5] + 27.0 * s6[10] - s6[15]) / 24.0;
-                    } else if (left) {
-                        const double *s1 = sc + m, *s2 = sc + 4 * 5 + m, *s3 = sc + 9 * 5 + m;
-                        if (l == 1) v = (-23.0 * s1[0] + 21.0 * s1[5] + 3.0 * s1[10] - 1.0 * s1[15]) / 24.0;
-                        else if (l == 2) v = (-22.0 * s2[0] + 17.0 * s2[5] + 9.0 * s2[10] - 5.0 * s2[15] + s2[20]) / 24.0;
-                        else v = (s3[0] - 27.0 * s3[5] + 27.0 * s3[10] - s3[15]) / 24.0;
+                    if (right || left) {
+                        v = section_difference(sc + m, right, right ? n - l : l - 1);
                     } else {
                         auto fa = [&](int hh) { return fr[(fslot(hh) * NLP + pl) * INV_FP + m]; };
                         v = flux_dxyz_at(fa, n, l);
@@ -388,6 +539,7 @@ __global__ void __launch_bounds__(INV_THREADS, INV_CTAS) k_rhs_invis(DevParams P
         fs = wrap(fs + len, FR);
         len = C;
     }
+    if (rest) nbad += inv_rest<dir, NFLUX>(&P, &F, &blocks[G.blk], groups + blockIdx.x, done, h0, C, smem, secf, sec);
     if (nbad) atomicAdd(&err[ERR_ROE], nbad);
 }
 

@@ -325,12 +325,54 @@ __device__ __forceinline__ double recip_sqrt(double x) {
     return fma(y, e * fma(e, 0.375, 0.5), y);
 }
 
-// flux_Roe (flux.f90:116-244) for the FP64 residual: the central part with the
-// operations of the reference and in their order; what the jump multiplies with
-// short reciprocals and roots, and sqrt(rl rr) as rl sqrt(rr / rl).
+// flux_Roe (flux.f90:116-244) with its operations in their order, for the half nodes
+// that flux_roe leaves.  l, r: the left and the right state.  Returns 1 when c^2 <= 0.
+__device__ __forceinline__ int flux_roe_div(double gama, double efix, double nx, double ny, double nz, const double *l, const double *r, double *f) {
+    const double gama1 = gama - 1.0, gama2 = gama / gama1, nt = 0.0;
+    double dq[5], fs[5], h[2];
+#pragma unroll
+    for (int s = 0; s < 2; s++) {  // flux (Convect.f90:1245-1272) with getem (GasModel.f90:358-374), of the right state first
+        const double *p = s ? l : r;
+        const double v2 = p[1] * p[1] + p[2] * p[2] + p[3] * p[3], em = p[4] / gama1 + 0.5 * p[0] * v2;
+        const double cit = nx * p[1] + ny * p[2] + nz * p[3] + nt, ms = p[0] * cit;
+        const double g[5] = {ms, ms * p[1] + nx * p[4], ms * p[2] + ny * p[4], ms * p[3] + nz * p[4], (em + p[4]) * cit - p[4] * nt};
+#pragma unroll
+        for (int m = 0; m < 5; m++) fs[m] = s ? fs[m] + g[m] : g[m];
+        h[s] = gama2 * p[4] / p[0] + 0.5 * v2;
+    }
+#pragma unroll
+    for (int m = 0; m < 5; m++) dq[m] = r[m] - l[m];
+    const double rm = sqrt(l[0] * r[0]), rrl = sqrt(r[0] / l[0]), w = rrl + 1.0;
+    const double um = (l[1] + r[1] * rrl) / w, vm = (l[2] + r[2] * rrl) / w, wm = (l[3] + r[3] * rrl) / w, hm = (h[1] + h[0] * rrl) / w;
+    const double c2 = (hm - 0.5 * (um * um + vm * vm + wm * wm)) * gama1, c = sqrt(c2);
+    const double cta = um * nx + vm * ny + wm * nz + nt;
+    const double cgm = fmax(sqrt(nx * nx + ny * ny + nz * nz), SML_SSS), cgm1 = 1.0 / cgm;
+    nx = nx * cgm1;
+    ny = ny * cgm1;
+    nz = nz * cgm1;
+    const double ccgm = c * cgm, det = efix * cgm, det2 = det * det;
+    auto root = [det2](double x) { return sqrt(x * x + det2); };
+    const double l1 = root(fabs(cta - ccgm)), l4 = root(fabs(cta)), l5 = root(fabs(cta + ccgm));
+    const double rodcta = rm * (dq[1] * nx + dq[2] * ny + dq[3] * nz), cta1 = cta * cgm1;
+    const double dp_c2 = dq[4] / c2, rodctac = rodcta / c;
+    const double a1 = l4 * (dq[0] - dp_c2), a2 = l5 * (dp_c2 + rodctac) * 0.5, a3 = l1 * (dp_c2 - rodctac) * 0.5;
+    const double a4 = a1 + a2 + a3, a5 = c * (a2 - a3);
+    const double a6 = l4 * (rm * dq[1] - nx * rodcta), a7 = l4 * (rm * dq[2] - ny * rodcta), a8 = l4 * (rm * dq[3] - nz * rodcta);
+    f[0] = 0.5 * (fs[0] - a4);
+    f[1] = 0.5 * (fs[1] - (um * a4 + nx * a5 + a6));
+    f[2] = 0.5 * (fs[2] - (vm * a4 + ny * a5 + a7));
+    f[3] = 0.5 * (fs[3] - (wm * a4 + nz * a5 + a8));
+    f[4] = 0.5 * (fs[4] - (hm * a4 + cta1 * a5 + um * a6 + vm * a7 + wm * a8 - c2 * a1 / gama1));
+    return c2 <= 0.0 ? 1 : 0;
+}
+
+// flux_Roe for the FP64 residual: the central part with the operations of the reference
+// and in their order; what the jump multiplies with short reciprocals and roots, and
+// sqrt(rl rr) as rl sqrt(rr / rl).
 // gama1_1 = 1 / (gama - 1); same: ql equals qr, which leaves the central part.
-// Returns 1 when c^2 <= 0.
-__device__ __forceinline__ int flux_roe(const DevParams &P, double gama1_1, const double *ql, const double *qr, double nx,
+// Returns false, and no flux, where it is not finite or c^2 is not well above the
+// round-off of the enthalpy that it is the rest of: flux_roe_div.
+__device__ __forceinline__ bool flux_roe(const DevParams &P, double gama1_1, const double *ql, const double *qr, double nx,
                                              double ny, double nz, double nt, bool same, double *f) {
     const double gama = P.gama, gama1 = gama - 1.0, gama2 = gama / gama1;
     const double v2l = ql[1] * ql[1] + ql[2] * ql[2] + ql[3] * ql[3], v2r = qr[1] * qr[1] + qr[2] * qr[2] + qr[3] * qr[3];
@@ -346,18 +388,20 @@ __device__ __forceinline__ int flux_roe(const DevParams &P, double gama1_1, cons
         s[3] = (mr * qr[3] + nz * qr[4]) + (ml * ql[3] + nz * ql[4]);
         s[4] = ((er + qr[4]) * cr - qr[4] * nt) + ((el + ql[4]) * cl - ql[4] * nt);
     }
+    // what is not finite reaches the energy flux, by each of the other terms
+    auto finite = [](double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; };
+    const double rl1 = recip(ql[0]);
     if (same) {
 #pragma unroll
         for (int m = 0; m < 5; m++) f[m] = 0.5 * s[m];
-        return ql[4] / ql[0] <= 0.0 ? 1 : 0;
+        const double pr = ql[4] * rl1;
+        return pr > 1.0e-10 * fma(gama2, pr, 0.5 * v2l) && finite(f[4]);
     }
-    const double rl1 = recip(ql[0]);
     const double hl = fma(gama2, ql[4] * rl1, 0.5 * v2l), hr = fma(gama2, qr[4] * recip(qr[0]), 0.5 * v2r);
     const double rr = qr[0] * rl1, rrl = rr * recip_sqrt(rr), w = recip(rrl + 1.0), rm = ql[0] * rrl;
     const double um = fma(qr[1], rrl, ql[1]) * w, vm = fma(qr[2], rrl, ql[2]) * w, wm = fma(qr[3], rrl, ql[3]) * w,
                  hm = fma(hr, rrl, hl) * w;
     const double c2 = (hm - 0.5 * fma(um, um, fma(vm, vm, wm * wm))) * gama1;
-    const int bad = c2 <= 0.0 ? 1 : 0;
     const double c_1 = recip_sqrt(c2), c = c2 * c_1;
     const double cta = fma(um, nx, fma(vm, ny, wm * nz)) + nt;
     const double k2 = fmax(fma(nx, nx, fma(ny, ny, nz * nz)), SML_SSS * SML_SSS), cgm1 = recip_sqrt(k2), cgm = k2 * cgm1;
@@ -379,7 +423,7 @@ __device__ __forceinline__ int flux_roe(const DevParams &P, double gama1_1, cons
     f[2] = 0.5 * (s[2] - fma(vm, a4, fma(ny, a5, a7)));
     f[3] = 0.5 * (s[3] - fma(wm, a4, fma(nz, a5, a8)));
     f[4] = 0.5 * (s[4] - (fma(hm, a4, cta * cgm1 * a5) + fma(um, a6, fma(vm, a7, wm * a8)) - c2 * a1 * gama1_1));
-    return bad;
+    return c2 > 1.0e-10 * hm && finite(f[4]);
 }
 
 // the flux-vector splittings chosen by nflux (Convect.f90:12-46): 1
