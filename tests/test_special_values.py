@@ -68,3 +68,42 @@ def test_viscous(field):
 @pytest.mark.parametrize("field", ["r", "u", "p"])
 def test_inviscid(field, nscheme, nflux):
     _compare(field, (INF, float("nan"), 1e30, 1e60), POINTS, nscheme, nflux, 0)
+
+
+@pytest.mark.parametrize("form", ["clustered", "wide", "plane"])
+@pytest.mark.parametrize("field,value", [("p", -1.0), ("p", 0.0), ("p", INF), ("p", float("nan")), ("r", -1.0), ("r", 0.0), ("r", INF), ("r", float("nan")),
+                                         ("u", INF), ("u", float("nan")), ("dq1", INF), ("dq5", float("nan")), ("sra", INF)], ids=str)
+def test_sweeps(field, value, form, monkeypatch):
+    """A state that turned bad between the time step and the sweeps: what the sweeps
+    hand on from there is undefined, whatever form they take."""
+    from oracle.pyoracle import Oracle
+    from tests.helpers import perturbed
+    from wcns_b200 import cases
+    from wcns_b200.solver import FLAG_SWEEP_BY_PLANE, FLAG_SWEEP_WIDE, Wcns, WcnsError
+    if form == "clustered":
+        monkeypatch.setenv("WCNS_SWEEP_CLUSTER", "4")
+    dims = (13, 9, 8)
+    for point in ((6, 6, 7), (4, 5, 5)):
+        case = perturbed(cases.vortex_case(ni=13, nj=9, nk=8, nscheme=4, nflux=1))
+        g, o = Wcns(case, flags={"clustered": 0, "wide": FLAG_SWEEP_WIDE, "plane": FLAG_SWEEP_BY_PLANE}[form]), Oracle(case)
+        assert g.sweep_mode() == form
+        for gp, op in [("boundary_all", "boundary_all"), ("initial_q_dq_c_t", "initial_q_dq_c_t"), ("timestep_tgh", "timestep"),
+                       ("r_h_s_invis", "rhs_invis"), ("communicate_dq_npp", "communicate_dq")]:
+            getattr(g, gp)()
+            o.phase(op)
+        a = o.get(field, 1)
+        a[point] = value
+        g.set(field, 1, a)
+        o.set(field, 1, a)
+        try:
+            g.l_h_s_tgh()
+        except WcnsError:
+            with pytest.raises(RuntimeError):
+                o.phase("lhs")
+            continue
+        o.phase("lhs")
+        for f in DQ + ["r", "u", "v", "w", "p"]:
+            x, y = interior(g.get(f, 1), dims), interior(o.get(f, 1), dims)
+            np.testing.assert_array_equal(_kinds(x), _kinds(y), err_msg=f"{f} {point}")
+            ok = np.isfinite(y)
+            assert np.max(np.abs(x[ok] - y[ok]), initial=0.0) <= 1e-10 * np.max(np.abs(y[ok]), initial=0.0), (f, point)

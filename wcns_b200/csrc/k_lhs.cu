@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(PREP_THREADS) k_lhs_prep(DevParams P, DevField
             R[SR_COED] = F.f[F_COED][id];
 #pragma unroll
             for (int m = 0; m < 5; m++) R[SR_RHS + m] = F.f[F_DQ1 + m][id];  // store_rhs_nb (LHS.f90:1592-1613)
-            R[SR_U + 0] = um;
+            R[SR_U + 0] = sw_velocity(um, hint);
             R[SR_U + 1] = vm;
             R[SR_U + 2] = wm;
             R[SR_U + 3] = hint + 0.5 * (um * um + vm * vm + wm * wm);

@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(256, 4) k_wide_prep(DevParams P, DevFields F, 
         const double rm = F.f[F_R][id], um = F.f[F_U][id], vm = F.f[F_V][id], wm = F.f[F_W][id], pres = F.f[F_P][id];
         // total enthalpy, gettmhmgm_ns (GasModel.f90:411-426)
         const double hint = gama / (gama - 1.0) * pres / rm;
-        put(WP_UV, um, vm);
+        put(WP_UV, sw_velocity(um, hint), vm);
         put(WP_WH, wm, hint + 0.5 * (um * um + vm * vm + wm * wm));
 #pragma unroll
         for (int m = 0; m < 8; m += 2) put(WP_G01 + m / 2, F.f[F_KCX + m][id], F.f[F_KCX + m + 1][id]);

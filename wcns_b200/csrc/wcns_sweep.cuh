@@ -28,6 +28,13 @@
 
 namespace wcns {
 
+// The velocity as the terms take it.  The routine divides by the sound speed and its
+// square: where c^2 is not a positive number all its terms are undefined, and so they
+// are here, by way of theta.  hint = c^2 / (gama - 1)
+__device__ __forceinline__ double sw_velocity(double u, double hint) {
+    return hint > 0.0 && hint <= 1.7976931348623157e308 ? u : __longlong_as_double(0x7ff8000000000000LL);
+}
+
 // theta = g.V
 __device__ __forceinline__ double sw_theta(double gx, double gy, double gz, double u, double v, double w) {
     return fma(gz, w, fma(gy, v, gx * u));
