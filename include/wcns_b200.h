@@ -243,12 +243,14 @@ int wcns_get_shape(WcnsContext *ctx, int *shape);
 int wcns_device_name(WcnsContext *ctx, char *buf, int len);
 int wcns_set_shape(WcnsContext *ctx, const int *shape);
 /* Autotuner: times every candidate shape (clusters of 1, 2, 4, 8, 16 CTAs in
- * both lane modes; 4, 8, 16, 32 lines per CTA for each residual kernel) on
+ * both lane modes and the wide sweeps, where the blocks fit a cluster; 4, 8,
+ * 16, 32 lines per CTA for each residual kernel) on
  * the context's current state, reps timed runs each after one warm-up, with
  * the phase each shapes (the LU-SGS phase; the inviscid and the viscous
  * residual), keeps the fastest and returns it in shape[4]; ms[3] (may be
  * NULL) receives the best device ms of those three phases.  The state is
- * not changed (dq is restored).  Takes a few hundred phase runs. */
+ * not changed (dq is restored); an error leaves the sweeps as they were.
+ * Takes a few hundred phase runs. */
 int wcns_autotune(WcnsContext *ctx, int reps, int *shape, double *ms);
 
 /* Tangent and adjoint of the inviscid residual and of the LU-SGS operator

@@ -275,13 +275,15 @@ static void free_owned(WcnsContext *c, void *p) {
     cudaFree(p);
 }
 
-// Contexts whose blocks have at most this many hyperplanes sweep clustered by
-// default, the shape that they have always reported.  It is not the faster
-// form any more, but close: 0.149 against 0.129 ms per step on the small plate
-// (35 planes, eight blocks), and the autotuner chooses.  Above, the wide
-// sweeps are the default (33x17x9: 0.176 against 0.209 ms; 65x33x17: 0.34
-// against 0.57; the 228,888-point plate: 0.61 against 0.85; the 64-case batch:
-// 0.55 against 2.25).
+// Contexts whose blocks have at most this many hyperplanes sweep clustered until they
+// are tuned.  This is no measured crossover: the wide form is the faster one there too
+// (us per step, clustered and wide: vortex of 9x8x7 153 and 140, of 21x9x7 194 and 180;
+// the small plate, eight blocks of 35 planes, 248 and 237; the small channel, 24 blocks of 32
+// planes, 399 and 314).  It keeps what wcns_get_shape has always reported for small
+// grids, a cluster size, which tests/test_autotune.py holds on the small plate; the
+// autotuner takes the wide form.  Above, the wide sweeps are the default (us of prep and
+// sweeps, clustered and wide: 33x17x9 209 and 176; 65x33x17 570 and 340; the
+// 228,888-point plate 850 and 610; the 64-case batch 2250 and 550).
 constexpr int SWEEP_SMALL_PLANES = 35;
 
 static int wide_alloc_arrays(WcnsContext *c) {
@@ -411,7 +413,7 @@ static int build_line_tables(WcnsContext *c, int inv_cap, int vis_cap, int passe
                 // nodes, 128 / cmax lines to a CTA.  8 is the fastest where there are
                 // CTAs enough for the chip: loads across the lines are 128 contiguous
                 // bytes (inviscid, channel of 4.2 M points: 1135 us, and 1206, 1481,
-                // 1813, 2127 for 16, 32, 64, 128).  On fewer points a CTA's chain of
+                // 1813, 2127 for 16, 32, 64, 128: the prices below).  On fewer points a CTA's chain of
                 // chunks is what takes time, and longer chunks of fewer lines give
                 // more CTAs with shorter chains (vortex of 65x33x17 points: 85 us with
                 // 8, then 67, 52, 46, 42).  Cost of a choice: the CTAs' chunks, two

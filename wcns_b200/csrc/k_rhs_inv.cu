@@ -23,13 +23,13 @@
 //   - the nonlinear weights are formed over a common denominator: with
 //     E = (eps + IS)^2, w_k = C_k / E_k / sum(C / E) = C_k prod_{j != k} E_j / S,
 //     one division per state instead of six (124 cycles each, a dozen
-//     instructions).  E is between eps^2 = 1e-12 and q^4, so the products stay far
-//     inside the exponent range;
+//     instructions).  E is between eps^2 = 1e-12 and q^4, so the products stay inside
+//     the exponent range while q is below 1e37 (beyond, see the end);
 //   - a half node's two states are formed by the thread that evaluates its
 //     flux: the smoothness indicators are computed twice, but nothing of them
 //     goes through shared memory;
 //   - a reciprocal whose last bit does not matter takes five instructions
-//     (recip), a quotient that does, by a constant, three (div_by);
+//     (recip), a quotient that does, by a constant, six (div_by);
 //   - the code of the few half nodes near a flagged end is kept out of the way
 //     and in one copy for the five variables: unrolled it was as long as the
 //     rest, and a quarter of the warps' time went into instruction fetches;
@@ -38,11 +38,12 @@
 //     arithmetic and stores follow one another; a ring of a chunk and its halo
 //     leaves room for 16 lines.
 // Measured per step, with the closures unrolled and whole lines; the code above on
-// whole lines; now: channel (24 blocks, 4.2 M points, Roe, nscheme 41) 3540, 1511,
-// 1135 us; 64 small blocks (0.9 M points) 1543, 539, 470; one block of 121x75x51
-// points (nscheme 4) 347, 190, 167; the plate (0.23 M points) 265, 148, 116; one
-// vortex of 65x33x17 73, 57, 42.  Three, five, six CTAs per SM over the channel:
-// 1228, 1216, 1323 us; two of 256 threads with C = 16 1300.
+// whole lines; now, chunk lengths as build_line_tables picks them: channel (24 blocks,
+// 4.2 M points, Roe, nscheme 41) 3540, 1511, 1152 us; 64 small blocks (0.9 M points)
+// 1543, 539, 472; one block of 121x75x51 points (nscheme 4) 347, 190, 171; the plate
+// (0.23 M points) 265, 148, 118; one vortex of 65x33x17 73, 57, 46.  Three, five, six
+// CTAs per SM over the channel, where four took 1135: 1228, 1216, 1323 us; two of 256
+// threads with C = 16 1300.
 // The central part of the fluxes and the differences keep the reference's
 // operations and their order: where the flow is uniform they cancel to
 // round-off, which is compared.  The weights, and in the Roe flux all that is

@@ -123,8 +123,8 @@ void launch_node_derivatives(const LaunchCtx &c) {
 //     share a bank;
 //   - formulas of the ends run in their own threads, not for a warp's every line.
 // Measured with the node derivatives, per step: channel (24 blocks, 4.2 M points)
-// 3110 us before, 1370 now; 64 small blocks (0.9 M points) 872 and 393 us; the plate
-// (8 blocks, 0.23 M points) 217 and 117 us.  Other splits over the channel: C = 10
+// 3110 us before, 1365 now; 64 small blocks (0.9 M points) 872 and 389 us; the plate
+// (8 blocks, 0.23 M points) 217 and 119 us.  Other splits over the channel: C = 10
 // 1437 us, C = 16 with 256 threads 1541, 64 threads 1804, 96 registers with spills
 // 1948; a ring that prefetches one chunk more (and holds fewer warps) 1861.
 constexpr int VIS_NF = 24, VIS_PITCH = 26, VIS_FP = 4;

@@ -62,8 +62,8 @@ __device__ __forceinline__ double conv_flux(double u, double v, double w, double
 // convection; the viscosity it needs there is a field (viseq, written with the
 // derivatives of qke), not a division per half point; the powers are products, and the
 // sixth root a cube root of a square root.  The terms add up in the reference's order.
-// Channel (4.2 M points) with the derivatives: 574 us before, 453 now; 64 small blocks
-// (0.9 M points) 143 and 113 us.  Three CTAs of 256 per SM; two 504 us, four 475.
+// Channel (4.2 M points) with the derivatives: 574 us before, 461 now; 64 small blocks
+// (0.9 M points) 143 and 120 us.  Three CTAs of 256 per SM; two 504 us, four 475.
 __device__ void sa_rhs_point(const DevFields &F, const SaFields &S, const SaParams &P, const DevBlock &B, int id) {
     const double uc = __ldg(F.f[F_U] + id), vc = __ldg(F.f[F_V] + id), wc = __ldg(F.f[F_W] + id), ro = __ldg(F.f[F_R] + id);
     const double vtbar = S.qke[id], visc = __ldg(S.vis + id);
