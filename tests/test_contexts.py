@@ -132,3 +132,18 @@ def test_adjoint_operators_of_two_threads():
         for res in out[q][0]:
             for a, b in zip(res, out[q][0][0]):
                 np.testing.assert_array_equal(a, b)
+
+
+def test_tuning_restores_dq_while_the_default_stream_is_busy():
+    """The context's stream and the default stream do not wait for each other."""
+    import torch
+    from wcns_b200.solver import Wcns
+    g = Wcns(perturbed(cases.small_plate_case()))
+    g.step(1)
+    before = [g.get(f"dq{m}", nb) for nb in range(1, len(g.dims) + 1) for m in range(1, 6)]
+    torch.cuda._sleep(400_000_000)  # some 0.2 s
+    g.autotune(1)
+    torch.cuda.synchronize()
+    after = [g.get(f"dq{m}", nb) for nb in range(1, len(g.dims) + 1) for m in range(1, 6)]
+    for a, b in zip(before, after):
+        np.testing.assert_array_equal(a, b)

@@ -68,12 +68,16 @@ struct HBlock {
     std::vector<int> bcindex;
 };
 
+// The context's stream does not wait for the default stream, so that what is set up on
+// one must not be read on the other: every copy and memset of a context goes to its own
+// stream.  (A synchronous copy from pageable memory returns before its last part has
+// arrived, a memset or a copy within the device before it has begun.)
 template <class T>
-T *dev_upload(const std::vector<T> &v) {
+T *dev_upload(const std::vector<T> &v, cudaStream_t stream) {
     if (v.empty()) return nullptr;
     T *p = nullptr;
     if (cudaMalloc(&p, sizeof(T) * v.size()) != cudaSuccess ||
-        cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaMemcpyAsync(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream) != cudaSuccess) {
         cudaGetLastError();
         if (p) cudaFree(p);
         return nullptr;
@@ -137,7 +141,7 @@ struct WcnsContext {
     }
     template <class T>
     T *up(const std::vector<T> &v) {
-        T *p = dev_upload(v);
+        T *p = dev_upload(v, stream);
         if (p) owned.push_back(p);
         else if (!v.empty()) upload_failed = true;
         return p;
@@ -301,10 +305,10 @@ static int wide_alloc_arrays(WcnsContext *c) {
     const size_t ring = (size_t)16 * WIDE_UNITS * A.ringn * A.nkmax * std::max(1, A.nbnd), fl = sizeof(unsigned) * (size_t)(A.nbnd + 1);
     CK(cudaMalloc(&A.ring, ring));
     c->owned.push_back(A.ring);
-    CK(cudaMemset(A.ring, 0, ring));
+    CK(cudaMemsetAsync(A.ring, 0, ring, c->stream));
     CK(cudaMalloc(&A.flags, fl));
     c->owned.push_back(A.flags);
-    CK(cudaMemset(A.flags, 0, fl));
+    CK(cudaMemsetAsync(A.flags, 0, fl, c->stream));
     A.epoch = A.flags + A.nbnd;
     if (c->sa_pool) {  // the model's scalar sweeps run on the wide chunks too
         CK(cudaMalloc(&A.sa, sizeof(double2) * WIDE_SA_PAIRS * (size_t)A.n));
@@ -342,7 +346,7 @@ static int pm_alloc(WcnsContext *c) {
         set_err("device allocation of the sweep arrays failed");
         return WCNS_ERR_CUDA;
     }
-    CK(cudaMemset(c->pm_pool, 0, pmbytes));
+    CK(cudaMemsetAsync(c->pm_pool, 0, pmbytes, c->stream));
     c->pm_bytes = pmbytes;
     for (int m = 0; m < 5; m++) c->PM.dq[m] = c->pm_pool + (size_t)m * c->total_pm;
     c->PM.dq_stride = c->total_pm;
@@ -760,7 +764,7 @@ static int build_tables(WcnsContext *c) {
     c->owned.push_back(L.res_out);
     CK(cudaMalloc(&L.bad_count, sizeof(int) * nbk));
     c->owned.push_back(L.bad_count);
-    CK(cudaMemset(L.bad_count, 0, sizeof(int) * nbk));
+    CK(cudaMemsetAsync(L.bad_count, 0, sizeof(int) * nbk, c->stream));
     CK(cudaMalloc(&L.bad_list, sizeof(long long) * BAD_CAP * nbk));
     c->owned.push_back(L.bad_list);
     return 0;
@@ -768,9 +772,9 @@ static int build_tables(WcnsContext *c) {
 
 static int check_errors(WcnsContext *c) {
     int h[ERR_NSLOTS];
+    CK(cudaMemcpyAsync(h, c->d_err, sizeof h, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    CK(cudaMemcpy(h, c->d_err, sizeof h, cudaMemcpyDeviceToHost));
-    CK(cudaMemset(c->d_err, 0, sizeof h));
+    CK(cudaMemsetAsync(c->d_err, 0, sizeof h, c->stream));
     if (h[ERR_ROE]) {
         set_err(std::string(c->P.nflux == 2 ? "flux_vanleer: c^2 < 0" : "flux_Roe: c^2 <= 0") + " at " +
                 std::to_string(h[ERR_ROE]) + " half-node states");
@@ -886,7 +890,7 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
     // field pool
     size_t bytes = sizeof(double) * (size_t)F_NPOOL * (size_t)c->total;
     if (cudaMalloc(&c->pool, bytes) != cudaSuccess) { delete c; set_err("device allocation of the field pool failed"); return WCNS_ERR_CUDA; }
-    cudaMemset(c->pool, 0, bytes);
+    if (cudaMemsetAsync(c->pool, 0, bytes, c->stream) != cudaSuccess) { delete c; set_err("clearing of the field pool failed"); return WCNS_ERR_CUDA; }
     for (int f = 0; f < F_NPOOL; f++) c->F.f[f] = c->pool + (size_t)f * c->total;
     c->F.f[F_VIST] = nullptr;
     std::vector<DevBlock> hb(nblocks);
@@ -927,13 +931,13 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
     c->PM.csize = L.sweep_cluster;
     CK(cudaMalloc(&c->d_err, sizeof(int) * ERR_NSLOTS));
     c->owned.push_back(c->d_err);
-    CK(cudaMemset(c->d_err, 0, sizeof(int) * ERR_NSLOTS));
+    CK(cudaMemsetAsync(c->d_err, 0, sizeof(int) * ERR_NSLOTS, c->stream));
     L.err = c->d_err;
     // grid metrics on the device
     double *xyzd = nullptr, *work = nullptr;
     CK(cudaMalloc(&xyzd, sizeof(double) * 3 * (size_t)c->total));
     CK(cudaMalloc(&work, sizeof(double) * 13 * (size_t)c->total));
-    cudaMemset(xyzd, 0, sizeof(double) * 3 * (size_t)c->total);
+    CK(cudaMemsetAsync(xyzd, 0, sizeof(double) * 3 * (size_t)c->total, c->stream));
     std::vector<double> tmp;
     for (int b = 0; b < nblocks; b++) {
         const DevBlock &d = hb[b];
@@ -945,8 +949,8 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
                 for (int j = 1; j <= d.nj; j++)
                     for (int i = 1; i <= d.ni; i++)
                         tmp[gidx(d, i, j, k) - d.off] = src[(i - 1) + (size_t)d.ni * ((j - 1) + (size_t)d.nj * (k - 1))];
-            if (cudaMemcpy(xyzd + (size_t)q * c->total + d.off, tmp.data(), sizeof(double) * tmp.size(),
-                           cudaMemcpyHostToDevice) != cudaSuccess) {
+            if (cudaMemcpyAsync(xyzd + (size_t)q * c->total + d.off, tmp.data(), sizeof(double) * tmp.size(),
+                                cudaMemcpyHostToDevice, c->stream) != cudaSuccess) {
                 set_err("wcns_create: copy of the coordinates to the device failed");
                 cudaFree(xyzd);
                 cudaFree(work);
@@ -1210,7 +1214,7 @@ static int interior_copy(WcnsContext *c, int nfields, const int *fields, double 
         c->stage_fields = 0;
         CK(cudaMalloc(&c->stage, sizeof(double) * (size_t)nfields * pts));
         CK(cudaMalloc(&c->stage_first, sizeof(long long) * first.size()));
-        CK(cudaMemcpy(c->stage_first, first.data(), sizeof(long long) * first.size(), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(c->stage_first, first.data(), sizeof(long long) * first.size(), cudaMemcpyHostToDevice, c->stream));
         c->stage_fields = nfields;
     }
     long long pts = 0;
@@ -1270,7 +1274,7 @@ extern "C" int wcns_sa_setup(WcnsContext *c, const double *const *xyz, double ti
     if (!(timedt_turb > 0.0)) { set_err("wcns_sa_setup: timedt_turb must be positive"); return WCNS_ERR_ARGUMENT; }
     if (!c->sa_pool) {
         CK(cudaMalloc(&c->sa_pool, sizeof(double) * SA_NFIELDS * (size_t)c->total));
-        CK(cudaMemset(c->sa_pool, 0, sizeof(double) * SA_NFIELDS * (size_t)c->total));
+        CK(cudaMemsetAsync(c->sa_pool, 0, sizeof(double) * SA_NFIELDS * (size_t)c->total, c->stream));
         double *f[SA_NFIELDS];
         for (int q = 0; q < SA_NFIELDS; q++) f[q] = c->sa_pool + (size_t)q * c->total;
         c->SA = SaFields{f[0], f[1], f[2], f[3], f[4], {f[5], f[6], f[7]}, f[8]};
@@ -1329,8 +1333,8 @@ extern "C" int wcns_sa_setup(WcnsContext *c, const double *const *xyz, double ti
                 for (int j = 1; j <= d.nj; j++)
                     for (int i = 1; i <= d.ni; i++)
                         tmp[gidx(d, i, j, k) - d.off] = src[(i - 1) + (size_t)d.ni * ((j - 1) + (size_t)d.nj * (k - 1))];
-            cudaError_t e = cudaMemcpy(xyzd + (size_t)q * c->total + d.off, tmp.data(), sizeof(double) * tmp.size(),
-                                       cudaMemcpyHostToDevice);
+            cudaError_t e = cudaMemcpyAsync(xyzd + (size_t)q * c->total + d.off, tmp.data(), sizeof(double) * tmp.size(),
+                                            cudaMemcpyHostToDevice, c->stream);
             if (e != cudaSuccess) { cudaFree(xyzd); set_err(std::string("wcns_sa_setup: ") + cudaGetErrorString(e)); return WCNS_ERR_CUDA; }
         }
     }
@@ -1358,9 +1362,9 @@ extern "C" int wcns_sa_setup(WcnsContext *c, const double *const *xyz, double ti
     int *wranged = nullptr;
     {
         cudaError_t e = cudaMalloc(&wranged, sizeof(int) * wrange.size());
-        if (e == cudaSuccess) e = cudaMemcpy(wranged, wrange.data(), sizeof(int) * wrange.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(wranged, wrange.data(), sizeof(int) * wrange.size(), cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess && !wall.empty()) e = cudaMalloc(&walld, sizeof(double) * wall.size());
-        if (e == cudaSuccess && !wall.empty()) e = cudaMemcpy(walld, wall.data(), sizeof(double) * wall.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && !wall.empty()) e = cudaMemcpyAsync(walld, wall.data(), sizeof(double) * wall.size(), cudaMemcpyHostToDevice, c->stream);
         if (e != cudaSuccess) {
             cudaFree(xyzd); cudaFree(walld); cudaFree(wranged);
             set_err(std::string("wcns_sa_setup: ") + cudaGetErrorString(e));
@@ -1825,7 +1829,7 @@ extern "C" int wcns_autotune(WcnsContext *c, int reps, int *shape, double *ms) {
     } copy;
     CK(cudaMalloc(&copy.p, bytes));
     const double *saved = copy.p;
-    CK(cudaMemcpy(copy.p, c->F.f[F_DQ1], bytes, cudaMemcpyDeviceToDevice));
+    CK(cudaMemcpyAsync(copy.p, c->F.f[F_DQ1], bytes, cudaMemcpyDeviceToDevice, c->stream));
     drop_graph(c);
     int best[4];
     wcns_get_shape(c, best);
@@ -1849,8 +1853,10 @@ extern "C" int wcns_autotune(WcnsContext *c, int reps, int *shape, double *ms) {
         best_ms[vis ? 2 : 1] = tbest;
     }
     if (!rc) rc = build_line_tables(c, best[2], best[3]);
-    cudaMemcpy(c->F.f[F_DQ1], saved, bytes, cudaMemcpyDeviceToDevice);
+    const cudaError_t back = cudaMemcpyAsync(c->F.f[F_DQ1], saved, bytes, cudaMemcpyDeviceToDevice, c->stream);
+    cudaStreamSynchronize(c->stream);  // before the copy goes
     if (rc) return rc;
+    CK(back);
     CK(cudaGetLastError());
     for (int q = 0; q < 4; q++) shape[q] = best[q];
     if (ms)
@@ -1876,7 +1882,7 @@ static int adj_ready(WcnsContext *c, const char *who) {
         setup_adj_attrs();
         const size_t bytes = sizeof(double) * 5 * (size_t)WCNS_ADJ_NSLOTS * (size_t)c->total;
         CK(cudaMalloc(&c->adj_pool, bytes));
-        CK(cudaMemset(c->adj_pool, 0, bytes));
+        CK(cudaMemsetAsync(c->adj_pool, 0, bytes, c->stream));
         // the records of the LU-SGS operator, unless they would take more than a
         // quarter of what is free: it goes plane by plane without them
         size_t free_b = 0, all_b = 0;
