@@ -15,7 +15,8 @@ STATE = ("r", "u", "v", "w", "p")
 
 
 class Hog:
-    """Device memory taken down to `leave` bytes (0: whatever the allocator still gives)."""
+    """All device memory but `leave` bytes (0: all that the allocator gives): chunks of
+    2 MB are set aside, the rest is taken, and the chunks are given back."""
 
     def __init__(self, leave=0):
         import torch
@@ -25,19 +26,23 @@ class Hog:
         self.held = []
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
-        top = torch.cuda.mem_get_info()[0] - leave
+        aside = [self._take(2 << 20) for _ in range(leave // (2 << 20))]
         size = 1 << 36
-        while size >= (512 if leave == 0 else 1 << 21):
-            if leave and size > top:
+        while size >= (2 << 20 if leave else 512):
+            p = self._take(size)
+            if p is None:
                 size >>= 1
-                continue
-            p = ctypes.c_void_p()
-            if self.rt.cudaMalloc(ctypes.byref(p), size) == 0:
-                self.held.append(p)
-                top -= size
             else:
-                self.rt.cudaGetLastError()
-                size >>= 1
+                self.held.append(p)
+        for p in aside:
+            self.rt.cudaFree(p)
+
+    def _take(self, size):
+        p = ctypes.c_void_p()
+        if self.rt.cudaMalloc(ctypes.byref(p), size) == 0:
+            return p
+        self.rt.cudaGetLastError()
+        return None
 
     def __enter__(self):
         return self
