@@ -120,3 +120,27 @@ def test_autotune_keeps_only_the_arrays_of_the_form_it_takes():
     assert before - _free() < (100 if g.sweep_mode() == "wide" else 500) << 20
     g.set_shape([0, 0] + g.shape[2:])
     assert before - _free() < 100 << 20
+
+
+def test_a_context_that_finds_no_memory_leaves_none_taken():
+    """Room for the field pool (281 MB), the residual's buffers (47) or the sweeps'
+    records, but not for all of them and the metrics' (75): an error, the memory
+    back, and no error left over for the next call of another context."""
+    from wcns_b200.solver import Wcns, WcnsError
+    small = perturbed(cases.small_plate_case())
+    big = cases.vortex_case(ni=121, nj=75, nk=51)
+    other, ref = Wcns(small), Wcns(small)
+    other.step(1), ref.step(1)
+    Wcns(big).close()  # what the library keeps from a first use is there
+    before = _free()
+    kept = Wcns(big)
+    all_but_metrics = (before - _free() >> 20) + 40
+    kept.close()
+    for room in (40, 300, 360, all_but_metrics):
+        with Hog(leave=room << 20):
+            before = _free()
+            with pytest.raises(WcnsError):
+                Wcns(big)
+            assert before - _free() < 8 << 20, room
+        _check(other, ref)
+    Wcns(big).close()

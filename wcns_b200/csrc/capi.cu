@@ -129,6 +129,7 @@ struct WcnsContext {
             if (L.ev_join[q]) cudaEventDestroy(L.ev_join[q]);
         }
         if (L.ev_fork) cudaEventDestroy(L.ev_fork);
+        delete[] L.hblocks;
         for (void *p : owned) cudaFree(p);
         if (pool) cudaFree(pool);
         if (pm_pool) cudaFree(pm_pool);
@@ -799,18 +800,14 @@ static void set_block_freestream(DevBlock &d, const DevParams &P, double moo) {
 }
 
 // ---------------------------------------------------------------------------
-extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, const double *const *xyz, int nregions,
-                           const int *regions, WcnsContext **out) {
-    if (!prm || nblocks < 1 || !dims || !xyz || !out || (nregions > 0 && !regions)) {
-        set_err("wcns_create: invalid argument");
-        return WCNS_ERR_ARGUMENT;
-    }
+// fills the context in; what it has when an error is returned goes with it
+static int create_context(WcnsContext *c, const WcnsParams *prm, int nblocks, const int *dims, const double *const *xyz, int nregions,
+                          const int *regions) {
     if (prm->nscheme != 4 && prm->nscheme != 41 && prm->nscheme != 42) { set_err("nscheme must be 4, 41 or 42"); return WCNS_ERR_UNSUPPORTED; }
     if (prm->nflux < 1 || prm->nflux > 3) { set_err("nflux must be 1 (Steger-Warming), 2 (Van Leer) or 3 (Roe)"); return WCNS_ERR_UNSUPPORTED; }
     if (prm->nvis != 0 && prm->nvis != 1) { set_err("nvis must be 0 or 1"); return WCNS_ERR_ARGUMENT; }
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) { set_err("no CUDA device"); return WCNS_ERR_CUDA; }
-    WcnsContext *c = new WcnsContext();
     c->prm = *prm;
     // derived constants (init_inflow PreProcess.f90:968-1113; read_perfect_gasmodel GasModel.f90:184-217)
     const double PAI = 3.14159265;
@@ -851,7 +848,7 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
         d.ni = dims[3 * b];
         d.nj = dims[3 * b + 1];
         d.nk = dims[3 * b + 2];
-        if (d.ni < 2 || d.nj < 2 || d.nk < 2) { delete c; set_err("block dimensions must be >= 2"); return WCNS_ERR_ARGUMENT; }
+        if (d.ni < 2 || d.nj < 2 || d.nk < 2) { set_err("block dimensions must be >= 2"); return WCNS_ERR_ARGUMENT; }
         d.gx = d.ni + 6;
         d.gy = d.nj + 6;
         d.gz = d.nk + 6;
@@ -867,7 +864,7 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
     c->total = off;
     for (int r = 0; r < nregions; r++) {
         const int *rr = regions + 16 * r;
-        if (rr[0] < 1 || rr[0] > nblocks) { delete c; set_err("BC region block number out of range"); return WCNS_ERR_ARGUMENT; }
+        if (rr[0] < 1 || rr[0] > nblocks) { set_err("BC region block number out of range"); return WCNS_ERR_ARGUMENT; }
         HReg R;
         for (int m = 0; m < 3; m++) {
             R.raw_s_st[m] = rr[1 + 2 * m];
@@ -881,16 +878,15 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
         c->blk[rr[0] - 1].regs.push_back(R);
     }
     int rc = analyze(c);
-    if (rc) { delete c; return rc; }
+    if (rc) return rc;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
-        delete c;
         set_err("cudaStreamCreate failed");
         return WCNS_ERR_CUDA;
     }
     // field pool
     size_t bytes = sizeof(double) * (size_t)F_NPOOL * (size_t)c->total;
-    if (cudaMalloc(&c->pool, bytes) != cudaSuccess) { delete c; set_err("device allocation of the field pool failed"); return WCNS_ERR_CUDA; }
-    if (cudaMemsetAsync(c->pool, 0, bytes, c->stream) != cudaSuccess) { delete c; set_err("clearing of the field pool failed"); return WCNS_ERR_CUDA; }
+    if (cudaMalloc(&c->pool, bytes) != cudaSuccess) { set_err("device allocation of the field pool failed"); return WCNS_ERR_CUDA; }
+    if (cudaMemsetAsync(c->pool, 0, bytes, c->stream) != cudaSuccess) { set_err("clearing of the field pool failed"); return WCNS_ERR_CUDA; }
     for (int f = 0; f < F_NPOOL; f++) c->F.f[f] = c->pool + (size_t)f * c->total;
     c->F.f[F_VIST] = nullptr;
     std::vector<DevBlock> hb(nblocks);
@@ -901,14 +897,12 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
     for (int q = 0; q < 2; q++) {
         if (cudaStreamCreateWithFlags(&L.side[q], cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&L.ev_join[q], cudaEventDisableTiming) != cudaSuccess) {
-            delete c;
             set_err("stream/event creation failed");
             return WCNS_ERR_CUDA;
         }
     }
     if (cudaEventCreateWithFlags(&L.ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaMalloc(&L.contrib, sizeof(double) * 10 * (size_t)c->total) != cudaSuccess) {
-        delete c;
         set_err("allocation of the residual contribution buffers failed");
         return WCNS_ERR_CUDA;
     }
@@ -925,16 +919,23 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
     }
     rc = build_tables(c);
     if (!rc) rc = c->uploads_done();
-    if (rc) { delete c; return rc; }
+    if (rc) return rc;
     if (!L.sweep_plane && !L.wide)
-        if (int rc2 = pm_alloc(c)) { delete c; return rc2; }
+        if (int rc2 = pm_alloc(c)) return rc2;
     c->PM.csize = L.sweep_cluster;
     CK(cudaMalloc(&c->d_err, sizeof(int) * ERR_NSLOTS));
     c->owned.push_back(c->d_err);
     CK(cudaMemsetAsync(c->d_err, 0, sizeof(int) * ERR_NSLOTS, c->stream));
     L.err = c->d_err;
     // grid metrics on the device
-    double *xyzd = nullptr, *work = nullptr;
+    struct Scratch {
+        double *xyz = nullptr, *work = nullptr;
+        ~Scratch() {
+            cudaFree(xyz);
+            cudaFree(work);
+        }
+    } scratch;
+    double *&xyzd = scratch.xyz, *&work = scratch.work;
     CK(cudaMalloc(&xyzd, sizeof(double) * 3 * (size_t)c->total));
     CK(cudaMalloc(&work, sizeof(double) * 13 * (size_t)c->total));
     CK(cudaMemsetAsync(xyzd, 0, sizeof(double) * 3 * (size_t)c->total, c->stream));
@@ -944,7 +945,7 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
         tmp.assign((size_t)d.gx * d.gy * d.gz, 0.0);
         for (int q = 0; q < 3; q++) {
             const double *src = xyz[3 * b + q];
-            if (!src) { set_err("missing coordinates"); cudaFree(xyzd); cudaFree(work); delete c; return WCNS_ERR_ARGUMENT; }
+            if (!src) { set_err("missing coordinates"); return WCNS_ERR_ARGUMENT; }
             for (int k = 1; k <= d.nk; k++)
                 for (int j = 1; j <= d.nj; j++)
                     for (int i = 1; i <= d.ni; i++)
@@ -952,9 +953,6 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
             if (cudaMemcpyAsync(xyzd + (size_t)q * c->total + d.off, tmp.data(), sizeof(double) * tmp.size(),
                                 cudaMemcpyHostToDevice, c->stream) != cudaSuccess) {
                 set_err("wcns_create: copy of the coordinates to the device failed");
-                cudaFree(xyzd);
-                cudaFree(work);
-                delete c;
                 return WCNS_ERR_CUDA;
             }
         }
@@ -962,9 +960,7 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
     double *xyzp[3] = {xyzd, xyzd + c->total, xyzd + 2 * c->total};
     launch_metrics(L, xyzp, work);
     cudaError_t e = cudaStreamSynchronize(c->stream);
-    cudaFree(xyzd);
-    cudaFree(work);
-    if (e != cudaSuccess) { set_err(std::string("metrics: ") + cudaGetErrorString(e)); delete c; return WCNS_ERR_CUDA; }
+    if (e != cudaSuccess) { set_err(std::string("metrics: ") + cudaGetErrorString(e)); return WCNS_ERR_CUDA; }
     // wall regions for the force integration, in block and region order
     {
         std::vector<DevWall> walls;
@@ -1003,7 +999,7 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
         if (L.nwall) {
             L.walls = c->up(walls);
             L.wall_xyz = c->up(wxyz);
-            if (int rc2 = c->uploads_done()) { delete c; return rc2; }
+            if (int rc2 = c->uploads_done()) return rc2;
             CK(cudaMalloc(&L.wall_pf, sizeof(double) * 3 * (size_t)npt));
             c->owned.push_back(L.wall_pf);
             CK(cudaMalloc(&L.wall_quad, sizeof(double) * 6 * (size_t)std::max(nq, 1LL)));
@@ -1012,14 +1008,28 @@ extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, 
             c->owned.push_back(L.wall_out);
         }
     }
-    *out = c;
+    return 0;
+}
+
+extern "C" int wcns_create(const WcnsParams *prm, int nblocks, const int *dims, const double *const *xyz, int nregions,
+                           const int *regions, WcnsContext **out) {
+    if (!prm || nblocks < 1 || !dims || !xyz || !out || (nregions > 0 && !regions)) {
+        set_err("wcns_create: invalid argument");
+        return WCNS_ERR_ARGUMENT;
+    }
+    auto c = std::make_unique<WcnsContext>();
+    if (const int rc = create_context(c.get(), prm, nblocks, dims, xyz, nregions, regions)) {
+        if (c->stream) cudaStreamSynchronize(c->stream);
+        cudaGetLastError();  // reported here: not again by the next call of another context
+        return rc;
+    }
+    *out = c.release();
     return 0;
 }
 
 extern "C" void wcns_destroy(WcnsContext *c) {
     if (!c) return;
     cudaStreamSynchronize(c->stream);
-    delete[] c->L.hblocks;
     delete c;
 }
 
